@@ -164,6 +164,17 @@ inline bool tf_origin(int n1, int n2, int *off1, int *off2, int *ntz, int *ntx) 
   return tf_origin_axis(n1, true, off1, ntz) && tf_origin_axis(n2, false, off2, ntx);
 }
 
+// A tile of the on-chip 2D kernel (onchip2d.cuh): one CTA.
+struct OcTile {
+  int shot;
+  int r0, c0;         // first padded row (multiple of 4) and column (even)
+  int TZ, TX;         // rows (multiple of 4) and columns (even) of the tile
+  int nb[4];          // neighbour CTA at the left, right, top, bottom; -1: none
+  int cell0, ncell;   // receiver cells of the tile
+  int nterm;          // injection terms kept in shared memory (0: in global memory)
+  int nline;          // edge lines
+};
+
 // Tensor maps of one shot for the pipelined 3D kernel (rank 3, one plane per
 // box): [2*buf + box], box 0 the 40 x 40 plane tile with halo, 1 the
 // 32 x 32 core tile.

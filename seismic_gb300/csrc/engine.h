@@ -37,6 +37,7 @@ struct sw_ctx {
   bool profiling = false;
   sw_stats stats{};
   RunOpts run_opts;
+  unsigned oc_epoch = 0;   // last packet epoch of the on-chip kernel's inbox
 };
 
 namespace swave {
@@ -99,6 +100,40 @@ struct PhaseShot {
   sw_prop_desc d;
   DevIO io;
 };
+
+// Plan of an on-chip 2D run (onchip.cu): launches of shots that are resident
+// together, their tiles, and per shot its receiver cells and scratch needs.
+struct OcGroup {
+  std::vector<int> members;
+  bool adj = false;
+  int tile0 = 0, ncta = 0, cap = 0;
+  int steps = 0, chunk = 0;   // steps of the longest member, steps per launch
+  size_t smem = 0, smem_v = 0;   // shared memory of a CTA, and with the velocity in it
+  bool vsm = false;
+};
+struct OcShotPlan {
+  int cell0 = 0, ncell = 0;
+  int nent = 0, M = 0, ncol = 0, nrow = 0, row0 = 0;   // injection terms (OcShot)
+  size_t idx0 = 0, idxm0 = 0, ell0 = 0;
+  bool image = false;
+};
+struct OcRun {
+  std::vector<OcGroup> groups;
+  std::vector<OcTile> tiles;
+  std::vector<int> cells, idx;
+  std::vector<OcShotPlan> shot;
+  size_t scratch = 0, inbox = 0;
+  char *d_scratch = nullptr;
+  void *d_inbox = nullptr, *d_tiles = nullptr, *d_cells = nullptr, *d_idx = nullptr,
+       *d_oc = nullptr;
+};
+// Whether a shot's phase can run on chip (its grid fits, and it uses nothing
+// that the on-chip kernel leaves out).
+bool oc_eligible(const sw_ctx *c, const PhaseShot &p, const RunOpts &opt);
+bool oc_plan(sw_ctx *c, const std::vector<PhaseShot> &shots, const std::vector<Geom> &G,
+             const std::vector<InjPlan> &inj, const std::vector<ExtPlan> &ext, OcRun &R);
+int oc_run(sw_ctx *c, const std::vector<ShotDev> &hs, const ShotDev *dshots, OcRun &R, bool rigid,
+           int *derr, uint64_t *launches);
 
 int fail(sw_ctx *c, int code, const char *fmt, ...);
 

@@ -81,6 +81,18 @@ bool encode_field_map3(CUtensorMap *m, const float *base, const Geom &g, int bz,
 int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
   const int nb = (int)shots.size();
   if (nb == 0) return SW_OK;
+  // Shots whose grid fits on chip run there (onchip.cu), the others through
+  // the per-step kernels.
+  bool oc = false;
+  {
+    std::vector<PhaseShot> on, off;
+    for (auto &p : shots) (oc_eligible(c, p, opt) ? on : off).push_back(p);
+    if (!on.empty() && !off.empty()) {
+      const int st = run_phases(c, on, opt);
+      return st ? st : run_phases(c, off, opt);
+    }
+    oc = off.empty();
+  }
   cudaStream_t s = c->stream;
   cudaError_t e;
   int st = SW_OK;
@@ -153,7 +165,6 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
     }
     if (!fits) tile.stream2d = 1;
   }
-  const bool t2 = (tile.stream2d == 2 || tile.stream2d == 3) && shots[0].d.g.twoD;
   // The pipelined 3D kernel packs (shot, z tile, x tile, y unit) into 7/8/8/8
   // bits; larger batches or grids use the streaming kernel.
   if (!shots[0].d.g.twoD && tile.stream3d == 2) {
@@ -206,6 +217,9 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
     bytes += rup(ext[b].ic.size() * 4) + 2 * rup(ext[b].wz.size() * 4);
     bytes += 2 * rup(std::max<size_t>(tx[b].size(), ty[b].size()) * 4 + 4);
   }
+  OcRun ocr;
+  oc = oc && oc_plan(c, shots, G, inj, ext, ocr);
+  const bool t2 = !oc && (tile.stream2d == 2 || tile.stream2d == 3) && shots[0].d.g.twoD;
   bytes += rup(nb * sizeof(ShotDev)) + 9 * rup((nb + 1) * sizeof(int)) + rup(sizeof(int));
   if (t2) {
     size_t ntile = 0;
@@ -690,7 +704,13 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
     return SW_OK;
   };
   uint64_t launches = 0;
-  if (opt.use_graph && nchunks > 1) {
+  if (oc) {
+    if ((st = oc_run(c, hs, dshots, ocr, opt.rigid, derr, &launches))) return st;
+    if (prof) {
+      c->stats.step_kernel_timed += (uint64_t)max_steps;
+      for (int q = 0; q < max_steps; ++q) c->stats.step_bytes += step_bytes_at(q);
+    }
+  } else if (opt.use_graph && nchunks > 1) {
     cudaGraph_t graph[2] = {nullptr, nullptr};
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
     const int ngraph = prof ? 2 : 1;   // [0] plain, [1] with event records
