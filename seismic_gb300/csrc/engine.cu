@@ -758,13 +758,13 @@ int sw_bandpass(sw_ctx *c, int ntr, int nt, float dt, float flo, float fhi, int 
   const float *din = (const float *)p;
   float *dout = (float *)dbuf(c, "bp_out", nb, &st);
   float *D = (float *)dbuf(c, "bp_d", (size_t)n * ntr * sizeof(float), &st);
-  float *T = (float *)dbuf(c, "bp_t", (size_t)n * ntr * sizeof(float), &st);
-  if (!dout || !D || !T) return st;
+  if (!dout || !D) return st;
+  int nl = 0;
   cudaError_t e = launch_bandpass(ntr, nt, npad, phase, lo.n, dc, hi.n, dc + 5 * lo.n,
                                   dc + 5 * (lo.n + hi.n), dc + 5 * (lo.n + hi.n) + npad, din,
-                                  dout, D, T, c->stream);
+                                  dout, D, c->stream, &nl);
   if (e != cudaSuccess) return cuda_fail(c, e, "band-pass");
-  c->stats.launches_total++;
+  c->stats.launches_total += nl;
   if ((st = download(c, traces, dout, nb))) return st;
   if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess) return cuda_fail(c, e, "band-pass");
   return SW_OK;

@@ -298,73 +298,142 @@ cudaError_t launch_rho_delp(const Geom &g, const float *rho_pad, float *delp, fl
 }
 
 // ---------------------------------------------------------------------------
-// Band-pass of traces (Bandpass.f90:89-149 with the filters of bandpass.c):
-// one thread per trace.  The trace is padded by npad samples at each end with
-// cosine-squared ramps from its end values, run through the low-cut and then
-// the high-cut cascade of second-order sections (forward, and for a
-// zero-phase filter again over the reversed samples 2..n-2), and its middle
-// nt samples are returned.  The work arrays are sample-major (sample i of
-// trace t at i*ntr + t) so that a warp's accesses coalesce.  Each section is
-// run in place: the old input samples and the new output samples it still
-// needs are carried in registers.  The first two outputs of every section
-// stay zero, as the reference's never-written work samples do.
+// Band-pass of traces (Bandpass.f90:89-149 with the filters of bandpass.c).
+// The trace is padded by npad samples at each end with cosine-squared ramps
+// from its end values, run through the low-cut and then the high-cut cascade
+// of second-order sections (forward, and for a zero-phase filter again over
+// the reversed samples 2..n-2), and its middle nt samples are returned.  The
+// work array D is sample-major (sample i of trace t at i*ntr + t), so that a
+// warp's accesses coalesce.
+//
+// The recursion is serial in time: one thread per trace, bound by its
+// instruction issue.  A pass runs up to four sections at once, section q one
+// sample behind section q-1, so that the sections' operations are
+// independent within an iteration and a sample costs one load and one store
+// for all of them; the inputs of the next eight samples are loaded ahead.
+// One thread per trace running one section at a time through memory took
+// 6.8 ms for 901 traces of 2223 samples (whole call, 14-pole zero phase).
+// The first two outputs of every section stay zero, as the reference's
+// never-written work samples do.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void bp_sections(float *X, int n, int ntr, int t, int ns,
-                                            const float *__restrict__ c) {
-  for (int q = 0; q < ns; ++q) {
-    const float c0 = c[5 * q], c1 = c[5 * q + 1], c2 = c[5 * q + 2], c3 = c[5 * q + 3],
-                c4 = c[5 * q + 4];
-    float xm2 = X[t], xm1 = X[(size_t)ntr + t], nm2 = 0.f, nm1 = 0.f;
-    for (int i = 2; i < n; ++i) {
-      const float xc = X[(size_t)i * ntr + t];
-      const float v = (((c0 * xc + c1 * xm1) + c2 * xm2) - c3 * nm1) - c4 * nm2;
-      X[(size_t)i * ntr + t] = v;
-      xm2 = xm1;
-      xm1 = xc;
-      nm2 = nm1;
-      nm1 = v;
-    }
-    X[t] = 0.f;
-    X[(size_t)ntr + t] = 0.f;
+__global__ void __launch_bounds__(256) k_bp_pad(int ntr, int nt, int npad, const float *lead,
+                                                const float *trail, const float *__restrict__ in,
+                                                float *__restrict__ D) {
+  __shared__ float tile[32][33];
+  const int n = nt + 2 * npad, t0 = 32 * blockIdx.x, i0 = 32 * blockIdx.y;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int r = w; r < 32; r += 8) {
+    const int t = t0 + r, i = i0 + lane;
+    if (t >= ntr || i >= n) continue;
+    const float *tr = in + (size_t)t * nt;
+    tile[r][lane] = i < npad ? tr[0] * lead[i]
+                    : i < npad + nt ? tr[i - npad] : tr[nt - 1] * trail[i - npad - nt];
   }
+  __syncthreads();
+  for (int r = w; r < 32; r += 8)
+    if (t0 + lane < ntr && i0 + r < n) D[(size_t)(i0 + r) * ntr + t0 + lane] = tile[lane][r];
 }
 
-__device__ __forceinline__ void bp_filter(float *D, float *T, int n, int ntr, int t, int ns,
-                                          const float *__restrict__ c, int phase) {
-  bp_sections(D, n, ntr, t, ns, c);
-  if (phase == 0) {
-    T[t] = 0.f;
-    T[(size_t)ntr + t] = 0.f;
-    for (int i = 2; i < n; ++i) T[(size_t)i * ntr + t] = D[(size_t)(n + 1 - i) * ntr + t];
-    bp_sections(T, n, ntr, t, ns, c);
-    for (int i = 2; i < n; ++i) D[(size_t)i * ntr + t] = T[(size_t)(n + 1 - i) * ntr + t];
-  }
+__global__ void __launch_bounds__(256) k_bp_cut(int ntr, int nt, int npad,
+                                                const float *__restrict__ D,
+                                                float *__restrict__ out) {
+  __shared__ float tile[32][33];
+  const int t0 = 32 * blockIdx.x, i0 = 32 * blockIdx.y;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int r = w; r < 32; r += 8)
+    if (t0 + lane < ntr && i0 + r < nt)
+      tile[r][lane] = D[(size_t)(npad + i0 + r) * ntr + t0 + lane];
+  __syncthreads();
+  for (int r = w; r < 32; r += 8)
+    if (t0 + r < ntr && i0 + lane < nt) out[(size_t)(t0 + r) * nt + i0 + lane] = tile[lane][r];
 }
 
-__global__ void k_bandpass(int ntr, int nt, int npad, int phase, int nlo, const float *clo,
-                           int nhi, const float *chi, const float *lead, const float *trail,
-                           const float *__restrict__ in, float *__restrict__ out, float *D,
-                           float *T) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+// NS sections over samples 2..n-1 of every trace, in place; with rev over
+// the reversed samples (sample i is D[n + 1 - i], before it zeros).
+template <int NS>
+__global__ void __launch_bounds__(32) k_bp_sections(int ntr, int n, int rev,
+                                                    const float *__restrict__ c, float *D) {
+  const int t = blockIdx.x * 32 + threadIdx.x;
   if (t >= ntr) return;
-  const int n = nt + 2 * npad;
-  const float *tr = in + (size_t)t * nt;
-  for (int i = 0; i < nt; ++i) D[(size_t)(npad + i) * ntr + t] = tr[i];
-  for (int j = 0; j < npad; ++j) {
-    D[(size_t)j * ntr + t] = tr[0] * lead[j];
-    D[(size_t)(n - npad + j) * ntr + t] = tr[nt - 1] * trail[j];
+  float cf[NS][5], xm1[NS], xm2[NS], nm1[NS], nm2[NS], v[NS];
+#pragma unroll
+  for (int q = 0; q < NS; ++q) {
+#pragma unroll
+    for (int m = 0; m < 5; ++m) cf[q][m] = c[5 * q + m];
+    xm1[q] = xm2[q] = nm1[q] = nm2[q] = v[q] = 0.f;
   }
-  if (nlo > 0) bp_filter(D, T, n, ntr, t, nlo, clo, phase);
-  if (nhi > 0) bp_filter(D, T, n, ntr, t, nhi, chi, phase);
-  float *o = out + (size_t)t * nt;
-  for (int i = 0; i < nt; ++i) o[i] = D[(size_t)(npad + i) * ntr + t];
+  if (!rev) {
+    xm2[0] = D[t];
+    xm1[0] = D[(size_t)ntr + t];
+  }
+  float *const first = rev ? D + (size_t)(n - 1) * ntr + t : D + 2 * (size_t)ntr + t;   // sample 2
+  const long long step = rev ? -(long long)ntr : (long long)ntr;
+  const int m = n - 2;   // samples
+  // Iteration k: section q takes sample k - q.
+  auto iterate = [&](int k, float x, bool check) {
+#pragma unroll
+    for (int q = NS - 1; q >= 0; --q) {
+      if (check && (k - q < 0 || k - q >= m)) continue;
+      const float xc = q ? v[q - 1] : x;
+      const float r = (((cf[q][0] * xc + cf[q][1] * xm1[q]) + cf[q][2] * xm2[q]) -
+                       cf[q][3] * nm1[q]) - cf[q][4] * nm2[q];
+      xm2[q] = xm1[q];
+      xm1[q] = xc;
+      nm2[q] = nm1[q];
+      nm1[q] = r;
+      v[q] = r;
+    }
+    if (k >= NS - 1) first[(k - (NS - 1)) * step] = v[NS - 1];
+  };
+  constexpr int U = 8;
+  int k = 0;
+  for (; k < NS - 1 && k < m; ++k) iterate(k, first[k * step], true);
+  float x[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) x[u] = k + u < m ? first[(k + u) * step] : 0.f;
+  for (; k + U <= m; k += U) {
+    float y[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) y[u] = k + U + u < m ? first[(k + U + u) * step] : 0.f;
+#pragma unroll
+    for (int u = 0; u < U; ++u) iterate(k + u, x[u], false);
+#pragma unroll
+    for (int u = 0; u < U; ++u) x[u] = y[u];
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (k + u < m) iterate(k + u, x[u], false);
+  for (k = m; k < m + NS - 1; ++k) iterate(k, 0.f, true);
+  if (!rev) D[t] = D[(size_t)ntr + t] = 0.f;
+}
+
+static void launch_bp_sections(int ntr, int n, int rev, int ns, const float *c, float *D,
+                               cudaStream_t s, int *nlaunch) {
+  const int g = (ntr + 31) / 32;
+  for (int q = 0; q < ns; q += 4) {
+    const float *cq = c + 5 * q;
+    switch (ns - q < 4 ? ns - q : 4) {
+      case 1: k_bp_sections<1><<<g, 32, 0, s>>>(ntr, n, rev, cq, D); break;
+      case 2: k_bp_sections<2><<<g, 32, 0, s>>>(ntr, n, rev, cq, D); break;
+      case 3: k_bp_sections<3><<<g, 32, 0, s>>>(ntr, n, rev, cq, D); break;
+      default: k_bp_sections<4><<<g, 32, 0, s>>>(ntr, n, rev, cq, D);
+    }
+    ++*nlaunch;
+  }
 }
 
 cudaError_t launch_bandpass(int ntr, int nt, int npad, int phase, int nlo, const float *clo,
                             int nhi, const float *chi, const float *lead, const float *trail,
-                            const float *in, float *out, float *D, float *T, cudaStream_t s) {
-  k_bandpass<<<(ntr + 127) / 128, 128, 0, s>>>(ntr, nt, npad, phase, nlo, clo, nhi, chi, lead,
-                                                trail, in, out, D, T);
+                            const float *in, float *out, float *D, cudaStream_t s,
+                            int *nlaunch) {
+  const int n = nt + 2 * npad, gx = (ntr + 31) / 32;
+  k_bp_pad<<<dim3(gx, (n + 31) / 32), 256, 0, s>>>(ntr, nt, npad, lead, trail, in, D);
+  launch_bp_sections(ntr, n, 0, nlo, clo, D, s, nlaunch);
+  if (phase == 0) launch_bp_sections(ntr, n, 1, nlo, clo, D, s, nlaunch);
+  launch_bp_sections(ntr, n, 0, nhi, chi, D, s, nlaunch);
+  if (phase == 0) launch_bp_sections(ntr, n, 1, nhi, chi, D, s, nlaunch);
+  k_bp_cut<<<dim3(gx, (nt + 31) / 32), 256, 0, s>>>(ntr, nt, npad, D, out);
+  *nlaunch += 2;
   return cudaGetLastError();
 }
 
