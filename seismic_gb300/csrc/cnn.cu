@@ -6,27 +6,30 @@
 // Activations and gradients are BF16 in channel-group planes: the channel
 // count is rounded up to 16 (zeros above the layer's own count) and group g
 // of 8 channels is a plane [x][z][8] of the image (pixel p = x * nz + z), so
-// element (p, c) sits at ((c / 8) * npix + p) * 8 + c % 8.  One GEMM tile is
-// a 32 (z) x 4 (x) patch of 128 pixels; the 8-channel slice of a tap-shifted
-// patch is 4 contiguous 512-byte rows that land in shared memory as 128 rows
-// of 16 bytes - exactly one K column of core matrices of the tensor cores'
-// no-swizzle layout (umma.cuh) - and one tensor copy fetches the slices of
-// all channel groups of a tap (zero fill outside the image).
+// element (p, c) sits at ((c / 8) * npix + p) * 8 + c % 8.  A pixel of a
+// plane is 16 bytes: eight consecutive pixels of a column are one core matrix
+// of the tensor cores' no-swizzle layout (umma.cuh), at any 16-byte offset.
 //
 // * Convolution (forward, and the input gradient with mirrored taps and
 //   transposed weights): implicit GEMM D[pixel][n] = sum over (tap,
 //   channel) on tcgen05 (M = 128 pixels, N = 16 or 32 output channels,
-//   K = 9 Cs), persistent CTAs, two shared-memory stages fed by TMA one
-//   tile ahead, the accumulator in tensor memory.  The epilogue fuses the
-//   bias and the ReLU (hidden layers write BF16 activations only), or the
-//   ReLU derivative of the layer input (input gradient), or writes the FP32
-//   output of the last layer.
+//   K = 9 Cs).  A block is 24 (z) x 16 (x) pixels; one tensor copy brings it
+//   with its one-pixel border (26 x 18 pixels, every channel group, zero
+//   fill outside the image).  An M = 128 tile is 8 (z) x 16 (x): its core
+//   matrices are one column apart, so every tap is the same operand at
+//   another start address and nothing is copied per tap.  The epilogue
+//   fuses the bias and the ReLU (hidden layers write BF16 activations
+//   only), or the ReLU derivative of the layer input (input gradient), or
+//   writes the FP32 output of the last layer.
 // * Weight gradient: dW[tap, ci][co] = sum_p a[p + off(tap)][ci] dz[p][co]
-//   on tcgen05 with both operands MN-major (the same tensor copies; K runs
-//   over pixels), M = 128 rows of (tap, ci) plus one row of ones that gives
-//   the bias gradient, N = output channels; each persistent CTA
-//   accumulates its pixels in tensor memory and writes one partial sum,
-//   and the partials are added in CTA order (deterministic).
+//   on tcgen05 with both operands MN-major (K = the 16 pixels of a column
+//   run).  The columns of a 16 x 16 pixel block are stored one after the
+//   other, so the rows of one product are the channels of 4 (8) adjacent
+//   columns: the three dx taps (and columns that are not used); dz taps are
+//   start addresses.  The bias gradient is summed from the staged gradient
+//   by the warps that wait for the accumulators.  Each persistent CTA
+//   accumulates its pixels in tensor memory and writes one partial sum, and
+//   the partials are added in a fixed order (deterministic).
 //
 // FP32 master weights and Adam state; the BF16 GEMM copies of the weights
 // are rewritten in the tensor cores' layout after every update.
@@ -48,10 +51,7 @@ using namespace swave;
 namespace {
 
 constexpr int kMaxC = 32;                 // channels per layer
-constexpr int kTZ = 32, kTX = 4;          // pixel patch of one GEMM tile
-constexpr int kTile = kTZ * kTX;          // 128 pixels = GEMM M
-constexpr int kChunk = kTile * 16;        // one 8-channel slice: 2048 bytes
-constexpr int kWgradSlots = 28 * kMaxC * kMaxC;   // partial sums per CTA (27 taps + bias)
+constexpr int kTile = 128;                // GEMM M
 
 int r16(int c);
 // Stored channels of a tensor: a multiple of 16, so that one tap of a
@@ -68,25 +68,18 @@ __device__ __forceinline__ void cnn_expect_tx(unsigned long long *bar, unsigned 
                "r"(bytes)
                : "memory");
 }
-// Tensor copy of the 8-channel slice of channel group cg at pixels
-// z..z+31 x x..x+3 of plane y (global -> shared memory, on an mbarrier).
-// The map's innermost dimension is (z, channel) flattened, so its
-// coordinate 8 z is a multiple of 16 bytes for every z.
-__device__ __forceinline__ void cnn_tma4(void *dst, const CUtensorMap *map, int cg, int z, int x,
-                                         int y, unsigned long long *bar) {
+// Tensor copy (global -> shared memory, on an mbarrier) of the box at pixel
+// row z and coordinates c1..c3 of the map's other dimensions.  The innermost
+// dimension is (z, channel) flattened, so its coordinate 8 z is a multiple of
+// 16 bytes for every z.
+__device__ __forceinline__ void cnn_tma4(void *dst, const CUtensorMap *map, int z, int c1, int c2,
+                                         int c3, unsigned long long *bar) {
   asm volatile(
       "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(umma_su32(dst)),
-      "l"(reinterpret_cast<unsigned long long>(map)), "r"(8 * z), "r"(x), "r"(y), "r"(cg),
+      "l"(reinterpret_cast<unsigned long long>(map)), "r"(8 * z), "r"(c1), "r"(c2), "r"(c3),
       "r"(umma_su32(bar))
       : "memory");
-}
-// Offsets of tap t of a 3 x 3 (taps = 9) or 3 x 3 x 3 (taps = 27) kernel:
-// t = 9 (dy + 1) + 3 (dx + 1) + (dz + 1).
-__device__ __forceinline__ void tap_off(int t, int taps, int &dz, int &dx, int &dy) {
-  dz = t % 3 - 1;
-  dx = (t / 3) % 3 - 1;
-  dy = taps == 27 ? t / 9 - 1 : 0;
 }
 // Instruction descriptor with both operands MN-major (transposed).
 __host__ __device__ constexpr uint32_t umma_idesc_bf16_mn(int M, int N) {
@@ -138,16 +131,26 @@ __device__ __forceinline__ void cnn_bar_init(unsigned long long *bar, unsigned c
 //   D[p][n] = sum_{tap, c} in[p + s * off(tap)][c] * W[n][tap * Cs + c]
 // with s = +1 (forward) or -1 (input gradient) and zero padding outside
 // the image.  W: NP x kp BF16 in the tensor cores' K-major layout.  One
-// ring stage holds one kernel row (a dz, and a dy in 3D): a single tensor
-// copy of the patch shifted by dz and widened to 6 columns (x0 - 1 ..
-// x0 + 4), every channel group.  In a plane of that copy ([6 x][32 z][8])
-// the patch shifted by dx is the contiguous run of 128 rows from column
-// dx + 1, so the three dx taps are three A operands of the same stage
-// (3 Cs / 16 K = 16 steps).  Two accumulators in tensor memory let the
-// products of the next tile run while the epilogue reads the last one.
+// ring stage holds one plane (a dy in 3D) of a block with its border: a
+// single tensor copy of kBZ x kBX pixels, every channel group, column pitch
+// kPitch bytes.  The M = 128 tile m (rows z0 + 8 m .. + 7 of the 16 columns)
+// of tap (dz, dx) starts at column dx + 1, row 8 m + dz + 1: core matrices
+// kPitch apart along M and one plane apart along K.  Two sets of kMT
+// accumulators in tensor memory let the products of the next block run
+// while the epilogue reads the last one.
+// Bound by the shared-memory reads of A (4 KB per product of 128 x NP x 16:
+// N is only 32).  Three copies per 32 x 4 pixel tile, one per dz, moved 4.5x
+// the pixels through L2 and took 26 / 30 us (forward / input gradient, 32
+// channels, 301 x 901 pixels, cold L2); this takes 17 / 18 us, and 36 us
+// instead of about 95 on 601 x 1801 pixels.
 // ---------------------------------------------------------------------------
 enum { kFwdHidden = 0, kFwdLast = 1, kBwd = 2 };
-constexpr int kMaxRing = 32;
+constexpr int kMaxRing = 16;
+constexpr int kMT = 3;                             // M tiles of a block
+constexpr int kCZ = 8 * kMT, kCX = 16;             // pixels of a block
+constexpr int kBZ = kCZ + 2, kBX = kCX + 2;        // with the border
+constexpr int kPitch = kBZ * 16;                   // bytes of a column
+constexpr int kPlane = kBX * kPitch;               // bytes of a channel group
 
 struct ConvArgs {
   int Cs;                        // stored input channels (multiple of 16)
@@ -168,24 +171,24 @@ struct ConvArgs {
 };
 
 __host__ __device__ inline size_t conv_wbytes(int NP, int kp) { return ((size_t)NP * kp * 2 + 1023) / 1024 * 1024; }
-constexpr int kConvCols = kTX + 2;                 // copy width: the patch and its x halo
-constexpr int kConvPlane = kConvCols * kTZ * 16;   // bytes of one channel group in a stage
 size_t conv_smem_bytes(int NP, int kp, int Cs, int ring) {
-  return 1024 + conv_wbytes(NP, kp) + (size_t)ring * (Cs / 8) * kConvPlane;
+  return 1024 + conv_wbytes(NP, kp) + (size_t)ring * (Cs / 8) * kPlane;
 }
 
 template <int NP, int MODE>
-__global__ void __launch_bounds__(kWsThreads, 1)
+__global__ void __launch_bounds__(kWsThreads, 2)
     k_conv_tma(const __grid_constant__ CUtensorMap amap, const ConvArgs A) {
   extern __shared__ unsigned char cnn_smem[];
   __shared__ __align__(8) unsigned long long full[kMaxRing], empty[kMaxRing];
   __shared__ __align__(8) unsigned long long acc_full[2], acc_empty[2];
+  __shared__ float sbias[kMaxC];
   __shared__ unsigned tmem_base;
   __shared__ volatile int abort_flag;
   __shared__ volatile int mma_stages;             // stages the MMA warp has consumed
+  constexpr unsigned kCols = NP == 32 ? 256 : 128;   // 2 x kMT accumulators of NP columns
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int nst = A.taps / 3;                     // ring stages (kernel rows) per tile
-  const size_t sbytes = (size_t)(A.Cs / 8) * kConvPlane;   // one kernel row
+  const int nst = A.taps / 9;                     // ring stages (planes) per block
+  const size_t sbytes = (size_t)(A.Cs / 8) * kPlane;
   unsigned char *base = align1024(cnn_smem);
   unsigned char *sW = base;
   unsigned char *ring = base + conv_wbytes(NP, A.kp);
@@ -202,7 +205,9 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     abort_flag = 0;
     mma_stages = 0;
   }
-  if (warp == kMmaWarp) umma_alloc(&tmem_base, 64);
+  if (tid < kMaxC) sbias[tid] = MODE != kBwd && tid < A.nout ? A.bias[tid] : 0.f;
+  if (warp == kMmaWarp) umma_alloc(&tmem_base, kCols);
+#pragma unroll 6
   for (int q = tid; q < NP * A.kp / 8; q += kWsThreads)
     reinterpret_cast<uint4 *>(sW)[q] = reinterpret_cast<const uint4 *>(A.W)[q];
   umma_fence_smem();
@@ -212,24 +217,22 @@ __global__ void __launch_bounds__(kWsThreads, 1)
   const unsigned tmem = tmem_base;
   const int first = blockIdx.x, stride = gridDim.x;
   const int nmine = first < A.ntiles ? (A.ntiles - 1 - first) / stride + 1 : 0;
+  const int sgn = A.mirror ? -1 : 1;
   if (warp == kProducerWarp) {
     if (lane == 0) {
-      const int sgn = A.mirror ? -1 : 1;
       int q = 0;
       bool ok = true;
       for (int i = 0; i < nmine && ok; ++i) {
         const int t = first + i * stride;
-        const int z0 = (t % A.tiles_z) * kTZ, x0 = ((t / A.tiles_z) % A.tiles_x) * kTX;
+        const int z0 = (t % A.tiles_z) * kCZ, x0 = ((t / A.tiles_z) % A.tiles_x) * kCX;
         const int y0 = t / (A.tiles_z * A.tiles_x);
         for (int k = 0; k < nst; ++k, ++q) {
           const int slot = q % A.ring;
           if (q >= A.ring && !(ok = cnn_wait(&empty[slot], ((q / A.ring) - 1) & 1, &abort_flag)))
             break;
-          unsigned char *dst = ring + (size_t)slot * sbytes;
           cnn_expect_tx(&full[slot], (unsigned)sbytes);
-          // Kernel row k: dz = k % 3 - 1, dy = k / 3 - 1 (3D).
-          const int dz = k % 3 - 1, dy = A.taps == 27 ? k / 3 - 1 : 0;
-          cnn_tma4(dst, &amap, 0, z0 + sgn * dz, x0 - 1, y0 + sgn * dy, &full[slot]);
+          cnn_tma4(ring + (size_t)slot * sbytes, &amap, z0 - 1, x0 - 1,
+                   y0 + (nst == 3 ? sgn * (k - 1) : 0), 0, &full[slot]);
         }
       }
       if (!ok) {
@@ -245,33 +248,41 @@ __global__ void __launch_bounds__(kWsThreads, 1)
   } else if (warp == kMmaWarp) {
     if (lane == 0) {
       constexpr uint32_t idesc = umma_idesc_bf16(kTile, NP);
-      const unsigned sb = umma_su32(sW);
+      const int nh = A.Cs / 16;
+      const uint64_t bdesc = umma_smem_desc(umma_su32(sW), (NP / 8) * 128, 128);
       int q = 0, committed = -1;
       bool ok = true;
       for (int i = 0; i < nmine && ok; ++i) {
         const int acc = i & 1;
         if (i >= 2 && !(ok = cnn_wait(&acc_empty[acc], ((i >> 1) - 1) & 1, &abort_flag))) break;
         umma_fence_after();
-        const unsigned d = tmem + acc * NP;
+        const unsigned d = tmem + acc * kMT * NP;
         for (int k = 0; k < nst; ++k, ++q) {
           const int slot = q % A.ring;
           if (!(ok = cnn_wait(&full[slot], (q / A.ring) & 1, &abort_flag))) break;
           mma_stages = q + 1;
           umma_fence_after();
-          const unsigned sa = umma_su32(ring + (size_t)slot * sbytes);
-          const int dz = k % 3 - 1, dy = A.taps == 27 ? k / 3 - 1 : 0;
-          for (int dx = -1; dx <= 1; ++dx) {
-            // Tap of (dz, dx, dy); its A operand starts at column s dx + 1.
-            const int t = 9 * (dy + 1) + 3 * (dx + 1) + (dz + 1) - (A.taps == 27 ? 0 : 9);
-            const unsigned col = (unsigned)((A.mirror ? -dx : dx) + 1) * kTZ * 16;
-            for (int h = 0; h < A.Cs / 16; ++h) {
-              const int ks = t * (A.Cs / 16) + h;
-              const uint64_t ad = umma_smem_desc(sa + h * 2 * kConvPlane + col, kConvPlane, 128);
-              const uint64_t bd =
-                  umma_smem_desc(sb + ks * 2 * (NP / 8) * 128, (NP / 8) * 128, 128);
-              umma_bf16(d, ad, bd, idesc, k > 0 || dx > -1 || h > 0);
+          // Descriptors differ in their start address alone (16-byte units):
+          // one addition per product, the issuing thread's own instructions
+          // would otherwise take longer than the products.
+          const uint64_t ad0 =
+              umma_smem_desc(umma_su32(ring + (size_t)slot * sbytes), kPlane, kPitch);
+          uint64_t ad[3];   // by s dz + 1
+          ad[0] = ad0 + (1 - sgn);
+          ad[1] = ad0 + 1;
+          ad[2] = ad0 + (1 + sgn);
+          const uint64_t bd0 = bdesc + (uint64_t)(9 * k * nh) * (2 * NP);
+          for (int dz = 0; dz < 3; ++dz)
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) {
+              uint64_t a = ad[dz] + (uint64_t)((sgn * (dx - 1) + 1) * (kPitch / 16));
+              uint64_t b = bd0 + (uint64_t)((3 * dx + dz) * nh) * (2 * NP);
+              for (int h = 0; h < nh; ++h, a += 2 * kPlane / 16, b += 2 * NP) {
+                const bool more = k > 0 || dz > 0 || dx > 0 || h > 0;
+#pragma unroll
+                for (int m = 0; m < kMT; ++m) umma_bf16(d + m * NP, a + m * 8, b, idesc, more);
+              }
             }
-          }
           umma_commit(&empty[slot]);
         }
         if (!ok) break;
@@ -285,9 +296,28 @@ __global__ void __launch_bounds__(kWsThreads, 1)
       if (committed >= 0) umma_mbar_wait(&acc_full[committed & 1], (committed >> 1) & 1);
     }
   } else {
-    // Epilogue: thread = accumulator lane = pixel row of the tile.
+    // Epilogue: thread = accumulator lane = row of an M tile, pixel
+    // (z0 + 8 m + row % 8, x0 + row / 8).
+    const size_t npix = (size_t)A.nz * A.nx * A.ny;
     for (int i = 0; i < nmine; ++i) {
       const int acc = i & 1;
+      const int t = first + i * stride;
+      const int z0 = (t % A.tiles_z) * kCZ + (tid & 7);
+      const int x = ((t / A.tiles_z) % A.tiles_x) * kCX + (tid >> 3);
+      const int y = t / (A.tiles_z * A.tiles_x);
+      // The ReLU masks are loaded before the products are waited for.
+      uint4 mk[MODE == kBwd ? kMT : 1][MODE == kBwd ? NP / 8 : 1];
+      if (MODE == kBwd) {
+#pragma unroll
+        for (int m = 0; m < kMT; ++m)
+#pragma unroll
+          for (int g = 0; g < NP / 8; ++g)
+            mk[m][g] = z0 + 8 * m < A.nz && x < A.nx && 8 * g < A.cs_out
+                           ? *reinterpret_cast<const uint4 *>(
+                                 A.mask + ((size_t)g * npix + ((size_t)y * A.nx + x) * A.nz + z0 +
+                                           8 * m) * 8)
+                           : make_uint4(0u, 0u, 0u, 0u);
+      }
       bool ok = cnn_wait(&acc_full[acc], (i >> 1) & 1, &abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) {
@@ -298,24 +328,24 @@ __global__ void __launch_bounds__(kWsThreads, 1)
         break;
       }
       umma_fence_after();
-      float accv[NP];
-      const unsigned ta = tmem + ((unsigned)(warp * 32) << 16) + acc * NP;
-      umma_ld16(ta, accv);
-      if (NP == 32) umma_ld16(ta + 16, accv + 16);
-      umma_fence_before();
-      __syncwarp();
-      if (lane == 0) cnn_arrive(&acc_empty[acc]);
-      const int t = first + i * stride;
-      const int z = (t % A.tiles_z) * kTZ + (tid % kTZ);
-      const int x = ((t / A.tiles_z) % A.tiles_x) * kTX + tid / kTZ;
-      const int y = t / (A.tiles_z * A.tiles_x);
-      if (z < A.nz && x < A.nx) {
+      const unsigned ta = tmem + ((unsigned)(warp * 32) << 16) + acc * kMT * NP;
+#pragma unroll
+      for (int m = 0; m < kMT; ++m) {
+        float accv[NP];
+        umma_ld16(ta + m * NP, accv);
+        if (NP == 32) umma_ld16(ta + m * NP + 16, accv + 16);
+        if (m == kMT - 1) {
+          umma_fence_before();
+          __syncwarp();
+          if (lane == 0) cnn_arrive(&acc_empty[acc]);
+        }
+        const int z = z0 + 8 * m;
+        if (z >= A.nz || x >= A.nx) continue;
         const size_t p = ((size_t)y * A.nx + x) * A.nz + z;
-        const size_t npix = (size_t)A.nz * A.nx * A.ny;
         if (MODE == kFwdLast) {
 #pragma unroll
           for (int n = 0; n < NP; ++n)
-            if (n < A.nout) A.out32[p * A.nout + n] = accv[n] + A.bias[n];
+            if (n < A.nout) A.out32[p * A.nout + n] = accv[n] + sbias[n];
         } else {
 #pragma unroll
           for (int c0 = 0; c0 < NP; c0 += 8) {
@@ -324,11 +354,10 @@ __global__ void __launch_bounds__(kWsThreads, 1)
             if (MODE == kFwdHidden) {
 #pragma unroll
               for (int j = 0; j < 8; ++j)
-                v[j] = c0 + j < A.nout ? fmaxf(accv[c0 + j] + A.bias[c0 + j], 0.f) : 0.f;
+                v[j] = c0 + j < A.nout ? fmaxf(accv[c0 + j] + sbias[c0 + j], 0.f) : 0.f;
             } else {
-              const uint4 mk =
-                  *reinterpret_cast<const uint4 *>(A.mask + ((size_t)(c0 / 8) * npix + p) * 8);
-              const unsigned mw[4] = {mk.x, mk.y, mk.z, mk.w};
+              const uint4 mq = mk[MODE == kBwd ? m : 0][MODE == kBwd ? c0 / 8 : 0];
+              const unsigned mw[4] = {mq.x, mq.y, mq.z, mq.w};
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
                 const unsigned short bits = (unsigned short)(mw[j >> 1] >> (16 * (j & 1)));
@@ -347,57 +376,70 @@ __global__ void __launch_bounds__(kWsThreads, 1)
   umma_fence_before();
   __syncthreads();
   umma_fence_after();
-  if (warp == kMmaWarp) umma_dealloc(tmem, 64);
+  if (warp == kMmaWarp) umma_dealloc(tmem, kCols);
 }
 
 // ---------------------------------------------------------------------------
 // Weight and bias gradient of one layer on the tensor cores.
-//   D[m][co] = sum_p A[m][p] * dz[p][co],  m = tap * Csi + ci  (A[m][p] =
-//   a[p + off(tap)][ci]),  m = taps Csi: a row of ones (bias gradient).
-// Both operands MN-major: each 8-channel slice copied by TMA is one MN
-// group of 8 rows x 128 pixels (core matrices 128 bytes apart along K, MN
-// groups one 2048-byte slice apart).  One ring stage serves one M = 128
-// slice of the rows for one tile: its 16 row groups (activation slices,
-// the ones slice copied from a constant array, stale data for rows past
-// the end, never stored) and the tile's Cout / 8 gradient slices.  Each
-// CTA accumulates its tiles in tensor memory (one accumulator per M
-// slice) and writes one partial sum.
+//   dW[tap, ci][co] = sum_p a[p + off(tap)][ci] dz[p][co]
+// A ring stage holds a 16 x 16 pixel block of dz ([group][column][16 z]) and
+// one plane (dy) of the activations around it, column by column: 18 columns
+// of kWZ rows (z0 - 1 ..; 18 are used, 20 keep what follows 128-byte aligned),
+// each [group][row].  Eight-channel groups are then kWPitch bytes apart over
+// the groups of a column and on into the next column, so the 128 rows of a
+// product for output column c are the channels of columns c, c + 1, ...: row
+// dxi * Csi + ci belongs to dx = dxi - 1 (rows of dxi > 2 are not used).  K
+// is the column's 16 pixels, dz a start address.  Accumulators: one per (dy,
+// dz).
+// Bound by the shared-memory reads of A, 4 KB per product; one copy of each
+// tap's own 32 x 4 pixel patch took 41 us (32 channels, 301 x 901 pixels, cold
+// L2), this takes 21 us.
 // ---------------------------------------------------------------------------
 struct WgradArgs {
   int Csi, Cin, Cso, Cout;
   int nz, nx, ny, taps, ntiles, tiles_z, tiles_x;
-  int nmma;                      // M = 128 slices: ceil((taps Csi + 8) / 128)
   int ring;                      // shared-memory stages (<= kMaxRing)
-  float *part;                   // [cta][10][kMaxC][kMaxC]
+  float *part;                   // [cta][tap or bias][kMaxC][kMaxC]
   int *err;
 };
-constexpr int kWgradStage = 20 * kChunk;   // 16 row groups + up to 4 gradient groups
+constexpr int kWB = 16;                      // pixels of a block along each axis
+constexpr int kWZ = 20, kWPitch = kWZ * 16;  // staged rows of a column, bytes per group
+constexpr int kWDz = kWB * kWB * 16;         // bytes of a channel group of dz
 
-size_t wgrad_smem_bytes(int ring) { return 1024 + (size_t)ring * kWgradStage; }
+// Columns of a stage: the rows of the last product reach this far (the ones
+// past the 18 copied hold stale data, which only unused rows read).
+__host__ __device__ inline int wgrad_cols(int Csi) { return kWB - 1 + kTile / Csi; }
+__host__ __device__ inline size_t wgrad_stage(int Csi, int Cso) {
+  return (size_t)wgrad_cols(Csi) * (Csi / 8) * kWPitch + (size_t)(Cso / 8) * kWDz;
+}
 
 template <int NPO>
 __global__ void __launch_bounds__(kWsThreads, 1)
     k_wgrad_umma(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap dmap,
-                 const __grid_constant__ CUtensorMap onemap, const WgradArgs A) {
+                 const WgradArgs A) {
   extern __shared__ unsigned char cnn_smem[];
   __shared__ __align__(8) unsigned long long full[kMaxRing], empty[kMaxRing], done;
   __shared__ unsigned tmem_base;
   __shared__ volatile int abort_flag;
   __shared__ volatile int mma_stages;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int G = A.taps * A.Csi / 8;               // activation groups; group G = ones
+  const int ndy = A.taps / 9;
+  const unsigned kCols = ndy == 1 ? 128 : 512;    // 3 ndy accumulators of NPO columns
+  const size_t abytes = (size_t)wgrad_cols(A.Csi) * (A.Csi / 8) * kWPitch;
+  const size_t sbytes = wgrad_stage(A.Csi, A.Cso);
+  const int colb = (A.Csi / 8) * kWPitch;         // bytes of a column
   unsigned char *ring = align1024(cnn_smem);
   if (tid == 0) {
     for (int q = 0; q < A.ring; ++q) {
       cnn_bar_init(&full[q], 1);
-      cnn_bar_init(&empty[q], 1);
+      cnn_bar_init(&empty[q], 1 + kEpiWarps);
     }
     cnn_bar_init(&done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     abort_flag = 0;
     mma_stages = 0;
   }
-  if (warp == kMmaWarp) umma_alloc(&tmem_base, 256);
+  if (warp == kMmaWarp) umma_alloc(&tmem_base, kCols);
   umma_fence_before();
   __syncthreads();
   umma_fence_after();
@@ -406,33 +448,20 @@ __global__ void __launch_bounds__(kWsThreads, 1)
   const int nmine = first < A.ntiles ? (A.ntiles - 1 - first) / stride + 1 : 0;
   if (warp == kProducerWarp) {
     if (lane == 0) {
-      const int ng = A.Csi / 8;
       int q = 0;
       bool ok = true;
       for (int i = 0; i < nmine && ok; ++i) {
         const int t = first + i * stride;
-        const int z0 = (t % A.tiles_z) * kTZ, x0 = ((t / A.tiles_z) % A.tiles_x) * kTX;
+        const int z0 = (t % A.tiles_z) * kWB, x0 = ((t / A.tiles_z) % A.tiles_x) * kWB;
         const int y0 = t / (A.tiles_z * A.tiles_x);
-        for (int j = 0; j < A.nmma; ++j, ++q) {
+        for (int k = 0; k < ndy; ++k, ++q) {
           const int slot = q % A.ring;
           if (q >= A.ring && !(ok = cnn_wait(&empty[slot], ((q / A.ring) - 1) & 1, &abort_flag)))
             break;
-          unsigned char *dst = ring + (size_t)slot * kWgradStage;
-          const int g1 = min(16 * j + 16, G + 1);
-          cnn_expect_tx(&full[slot], (unsigned)((g1 - 16 * j + A.Cso / 8) * kChunk));
-          // One tensor copy per tap (its ng channel-group slices; 16 is a
-          // multiple of ng), the ones slice, then the gradient's slices.
-          for (int g = 16 * j; g < g1; g += (g < G ? ng : 1)) {
-            unsigned char *gd = dst + (size_t)(g - 16 * j) * kChunk;
-            if (g < G) {
-              int dz, dx, dy;
-              tap_off(g / ng, A.taps, dz, dx, dy);
-              cnn_tma4(gd, &amap, 0, z0 + dz, x0 + dx, y0 + dy, &full[slot]);
-            } else {
-              cnn_tma4(gd, &onemap, 0, 0, 0, 0, &full[slot]);
-            }
-          }
-          cnn_tma4(dst + (size_t)16 * kChunk, &dmap, 0, z0, x0, y0, &full[slot]);
+          unsigned char *dst = ring + (size_t)slot * sbytes;
+          cnn_expect_tx(&full[slot], (unsigned)((kWB + 2) * colb + (A.Cso / 8) * kWDz));
+          cnn_tma4(dst + abytes, &dmap, z0, x0, y0, 0, &full[slot]);
+          cnn_tma4(dst, &amap, z0 - 1, 0, x0 - 1, y0 + (ndy == 3 ? k - 1 : 0), &full[slot]);
         }
       }
       if (!ok) {
@@ -449,21 +478,24 @@ __global__ void __launch_bounds__(kWsThreads, 1)
       int q = 0;
       bool ok = true, any = false;
       for (int i = 0; i < nmine && ok; ++i)
-        for (int j = 0; j < A.nmma; ++j, ++q) {
+        for (int k = 0; k < ndy; ++k, ++q) {
           const int slot = q % A.ring;
           if (!(ok = cnn_wait(&full[slot], (q / A.ring) & 1, &abort_flag))) break;
           mma_stages = q + 1;
           umma_fence_after();
-          const unsigned sa = umma_su32(ring + (size_t)slot * kWgradStage);
-          const unsigned sb = sa + 16 * kChunk;
-          // MN-major, no swizzle: the leading byte offset is the step
-          // between 8-row core-matrix groups along K (128 bytes here), the
-          // stride byte offset the step between 8-element groups along M / N
-          // (one 2048-byte slice).
+          const unsigned sa = umma_su32(ring + (size_t)slot * sbytes);
+          // MN-major, no swizzle: the leading byte offset is the step between
+          // the core matrices of 8 pixels along K (128 bytes), the stride
+          // byte offset the step between 8-channel groups along M / N.
+          uint64_t ad = umma_smem_desc(sa, 128, kWPitch);
+          uint64_t bd = umma_smem_desc(sa + (unsigned)abytes, 128, kWDz);
+          const unsigned d = tmem + 3 * k * NPO;
+#pragma unroll 4
+          for (int c = 0; c < kWB; ++c, ad += colb / 16, bd += kWB) {
+            const bool more = i > 0 || c > 0;
 #pragma unroll
-          for (int ks = 0; ks < kTile / 16; ++ks)
-            umma_bf16(tmem + j * NPO, umma_smem_desc(sa + ks * 256, 128, kChunk),
-                      umma_smem_desc(sb + ks * 256, 128, kChunk), idesc, i > 0 || ks > 0);
+            for (int dz = 0; dz < 3; ++dz) umma_bf16(d + dz * NPO, ad + dz, bd, idesc, more);
+          }
           umma_commit(&empty[slot]);
           any = true;
         }
@@ -475,29 +507,52 @@ __global__ void __launch_bounds__(kWsThreads, 1)
       else cnn_arrive(&done);
     }
   } else if (nmine > 0) {
-    // Epilogue: thread = accumulator lane = row (tap, ci) within a slice.
-    bool ok = cnn_wait(&done, 0, &abort_flag) && !abort_flag;
+    // While the products run: warp g sums channel group g of dz (once per
+    // block) over its pixels.
+    float bs[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    bool ok = true;
+    for (int q = 0; q < nmine * ndy && ok; ++q) {
+      const int slot = q % A.ring;
+      ok = __all_sync(0xffffffffu, cnn_wait(&full[slot], (q / A.ring) & 1, &abort_flag));
+      if (ok && q % ndy == 0 && warp < A.Cso / 8) {
+        const uint4 *g = reinterpret_cast<const uint4 *>(ring + (size_t)slot * sbytes + abytes +
+                                                         (size_t)warp * kWDz);
+#pragma unroll
+        for (int r = 0; r < kWB * kWB / 32; ++r) {
+          const uint4 v = g[lane + 32 * r];
+          const unsigned w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            bs[j] += __uint_as_float(j & 1 ? w[j >> 1] & 0xffff0000u : w[j >> 1] << 16);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) cnn_arrive(&empty[slot]);
+    }
+    // Epilogue: thread = accumulator lane = row dxi * Csi + ci.
+    ok = ok && cnn_wait(&done, 0, &abort_flag) && !abort_flag;
     ok = __all_sync(0xffffffffu, ok);
     umma_fence_after();
     if (ok) {
-      float *P = A.part + (size_t)blockIdx.x * kWgradSlots;
-      for (int j = 0; j < A.nmma; ++j) {
+      float *P = A.part + (size_t)blockIdx.x * (A.taps + 1) * kMaxC * kMaxC;
+      const int dxi = tid / A.Csi, ci = tid % A.Csi;
+      for (int j = 0; j < 3 * ndy; ++j) {
         float accv[NPO];
         const unsigned ta = tmem + ((unsigned)(warp * 32) << 16) + j * NPO;
         umma_ld16(ta, accv);
         if (NPO == 32) umma_ld16(ta + 16, accv + 16);
-        const int m = j * kTile + tid;
-        if (m < A.taps * A.Csi) {
-          const int tap = m / A.Csi, ci = m % A.Csi;
-          if (ci < A.Cin)
-#pragma unroll
-            for (int co = 0; co < NPO; ++co)
-              if (co < A.Cout) P[(size_t)tap * kMaxC * kMaxC + co * kMaxC + ci] = accv[co];
-        } else if (m == A.taps * A.Csi) {
+        const int tap = 9 * (j / 3) + 3 * dxi + j % 3;
+        if (dxi < 3 && ci < A.Cin) {
 #pragma unroll
           for (int co = 0; co < NPO; ++co)
-            if (co < A.Cout) P[(size_t)A.taps * kMaxC * kMaxC + co * kMaxC] = accv[co];
+            if (co < A.Cout) P[(size_t)tap * kMaxC * kMaxC + co * kMaxC + ci] = accv[co];
         }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        for (int o = 16; o > 0; o >>= 1) bs[j] += __shfl_xor_sync(0xffffffffu, bs[j], o);
+        if (lane == 0 && 8 * warp + j < A.Cout)
+          P[(size_t)A.taps * kMaxC * kMaxC + (8 * warp + j) * kMaxC] = bs[j];
       }
     } else if (lane == 0) {
       abort_flag = 1;
@@ -511,34 +566,57 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     // A give-up left products in flight: wait (bounded) for the last commit.
     if (abort_flag && lane == 0) umma_mbar_wait(&done, 0);
     __syncwarp();
-    umma_dealloc(tmem, 256);
+    umma_dealloc(tmem, kCols);
   }
 }
 
-// Sums the per-CTA partials in CTA order into the layer's gradient buffer
-// (FP32, [co][tap][ci] then bias[co]) - added to what it holds.  Block
-// `taps` is the bias.
-__global__ void k_wgrad_sum(const float *__restrict__ part, int nchunk, int Cout, int Cin,
-                            int taps, float *__restrict__ gw) {
-  const int tap = blockIdx.x, t = threadIdx.x;
-  const int co = t / kMaxC, ci = t % kMaxC;
-  if (co >= Cout || (tap == taps ? ci != 0 : ci >= Cin)) return;
+// Sums the per-CTA partials of every layer into the gradient buffer (FP32,
+// per layer [co][tap][ci] then bias[co]) - added to what it holds.  Block
+// (tap, co, layer), tap `taps` being the bias: 16 threads per input channel
+// take every sixteenth partial, then the 16 sums are added in order.
+constexpr int kSumW = 16, kMaxLayers = 16;
+struct SumArgs {
+  const float *part[kMaxLayers];
+  int nchunk, taps;
+  int Cin[kMaxLayers], Cout[kMaxLayers];
+  size_t off[kMaxLayers];
+  float *g;
+};
+__host__ __device__ inline size_t part_floats(int taps) {
+  return (size_t)(taps + 1) * kMaxC * kMaxC;   // of one CTA
+}
+__global__ void __launch_bounds__(kSumW * kMaxC) k_wgrad_sum(const SumArgs A) {
+  __shared__ float sh[kSumW][kMaxC];
+  const int tap = blockIdx.x, co = blockIdx.y, l = blockIdx.z;
+  const int ci = threadIdx.x % kMaxC, w = threadIdx.x / kMaxC;
+  const int Cin = A.Cin[l], Cout = A.Cout[l], taps = A.taps;
+  if (co >= Cout) return;
+  const bool use = tap == taps ? ci == 0 : ci < Cin;
+  const float *P = A.part[l] + (size_t)tap * kMaxC * kMaxC + co * kMaxC + ci;
   float s = 0.f;
-  for (int c = 0; c < nchunk; ++c) s += part[(size_t)c * kWgradSlots + tap * kMaxC * kMaxC + t];
+#pragma unroll 10
+  for (int c = w; c < A.nchunk; c += kSumW) s += use ? P[c * part_floats(taps)] : 0.f;
+  sh[w][ci] = s;
+  __syncthreads();
+  if (w != 0 || !use) return;
+  for (int q = 1; q < kSumW; ++q) s += sh[q][ci];
+  float *gw = A.g + A.off[l];
   if (tap == taps) gw[(size_t)Cout * taps * Cin + co] += s;
   else gw[((size_t)co * taps + tap) * Cin + ci] += s;
 }
 
-// Planar FP32 channels (c, p) -> BF16 channel-group planes with Cs stored
-// channels (q = (g * npix + p) * 8 + c % 8).
-__global__ void k_pack_input(const float *__restrict__ in, int C, int Cs, int npix,
+// Planar FP32 channels (c, p) -> BF16 channel-group planes; block row y is
+// group y, a thread packs the 8 channels of one pixel.
+__global__ void k_pack_input(const float *__restrict__ in, int C, int npix,
                              __nv_bfloat16 *__restrict__ out) {
-  const long long n = (long long)Cs * npix;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
-       q += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(q / (8LL * npix)) * 8 + (int)(q % 8);
-    const long long p = (q / 8) % npix;
-    out[q] = __float2bfloat16(c < C ? in[(size_t)c * npix + p] : 0.f);
+  const int g = blockIdx.y;
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = 8 * g + j < C ? in[(size_t)(8 * g + j) * npix + p] : 0.f;
+    *reinterpret_cast<uint4 *>(out + ((size_t)g * npix + p) * 8) =
+        make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]),
+                   pack_bf16(v[6], v[7]));
   }
 }
 
@@ -548,7 +626,7 @@ __global__ void k_pack_input(const float *__restrict__ in, int C, int Cs, int np
 // (out - target)^2.
 __global__ void k_loss(const float *__restrict__ out, const float *__restrict__ tgt, int npix,
                        __nv_bfloat16 *__restrict__ db, double *__restrict__ part) {
-  __shared__ double red[256];
+  __shared__ double red[8];
   double s = 0.0;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
     const float e = out[p] - tgt[p];
@@ -557,13 +635,13 @@ __global__ void k_loss(const float *__restrict__ out, const float *__restrict__ 
         make_uint4(pack_bf16(e / (float)npix, 0.f), 0u, 0u, 0u);
     *reinterpret_cast<uint4 *>(db + ((size_t)npix + p) * 8) = make_uint4(0u, 0u, 0u, 0u);
   }
-  red[threadIdx.x] = s;
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) s += red[w];
+    part[blockIdx.x] = s;
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
 // Adam on the FP32 master weights.
@@ -605,17 +683,23 @@ __global__ void k_weights_bf16(const float *__restrict__ w, int Cout, int Cin, i
 int nblk(long long n) { return (int)std::min<long long>(4096, (n + 255) / 256); }
 
 // BF16 tensor map over Cs / 8 channel-group planes: dimensions (8 nz: z
-// and the 8 channels flattened, nx, ny, Cs / 8), box 8 kTZ x cols x 1 x
-// planes (cols rows of 512 bytes per plane), zero fill outside.
+// and the 8 channels flattened, nx, ny, Cs / 8), box rows x cols pixels of
+// one plane, every group; zero fill outside.  by_column: the groups come
+// before the columns (dimensions 8 nz, Cs / 8, nx, ny), so that a box lands
+// column by column.
 bool encode_act_map(CUtensorMap *m, const __nv_bfloat16 *base, int Cs, int nz, int nx, int ny,
-                    int planes, int cols = kTX) {
+                    int rows, int cols, bool by_column = false) {
   PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
   if (!enc) return false;
-  const cuuint64_t dims[4] = {(cuuint64_t)nz * 8, (cuuint64_t)nx, (cuuint64_t)ny,
-                              (cuuint64_t)Cs / 8};
-  const cuuint64_t strides[3] = {(cuuint64_t)nz * 16, (cuuint64_t)nz * nx * 16,
-                                 (cuuint64_t)nz * nx * ny * 16};
-  const cuuint32_t box[4] = {8 * kTZ, (cuuint32_t)cols, 1, (cuuint32_t)planes};
+  const cuuint64_t col = (cuuint64_t)nz * 16, plane = col * nx, grp = plane * ny,
+                   G = (cuuint64_t)Cs / 8;
+  const cuuint64_t d0[4] = {(cuuint64_t)nz * 8, (cuuint64_t)nx, (cuuint64_t)ny, G},
+                   d1[4] = {(cuuint64_t)nz * 8, G, (cuuint64_t)nx, (cuuint64_t)ny};
+  const cuuint64_t s0[3] = {col, plane, grp}, s1[3] = {grp, col, plane};
+  const cuuint32_t b0[4] = {8 * (cuuint32_t)rows, (cuuint32_t)cols, 1, (cuuint32_t)G},
+                   b1[4] = {8 * (cuuint32_t)rows, (cuuint32_t)G, (cuuint32_t)cols, 1};
+  const cuuint64_t *dims = by_column ? d1 : d0, *strides = by_column ? s1 : s0;
+  const cuuint32_t *box = by_column ? b1 : b0;
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16 *>(base), dims,
              strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -643,22 +727,22 @@ cudaError_t launch_big(K kernel, int grid, size_t smem, cudaStream_t s, const CU
 cudaError_t launch_conv(int dev, int mode, int NP, const __nv_bfloat16 *in, int Cs, int nz, int nx,
                         int ny, int taps, ConvArgs a, cudaStream_t s) {
   CUtensorMap m;
-  if (!encode_act_map(&m, in, Cs, nz, nx, ny, Cs / 8, kConvCols)) return cudaErrorInvalidValue;
+  if (!encode_act_map(&m, in, Cs, nz, nx, ny, kBZ, kBX)) return cudaErrorInvalidValue;
   a.Cs = Cs;
   a.nz = nz;
   a.nx = nx;
   a.ny = ny;
   a.taps = taps;
   a.kp = r16(taps * Cs);
-  a.tiles_z = (nz + kTZ - 1) / kTZ;
-  a.tiles_x = (nx + kTX - 1) / kTX;
+  a.tiles_z = (nz + kCZ - 1) / kCZ;
+  a.tiles_x = (nx + kCX - 1) / kCX;
   a.ntiles = a.tiles_z * a.tiles_x * ny;
-  // A ring of about 110 KB per CTA (two CTAs per SM); stages of one tap.
-  const size_t stage = (size_t)(Cs / 8) * kConvPlane;
-  a.ring = (int)std::max<size_t>(
-      2, std::min<size_t>(kMaxRing, (110u * 1024u - 1024u - conv_wbytes(NP, a.kp)) / stage));
+  // Two CTAs per SM where at least two stages fit beside the weights, else
+  // one with a longer ring.
+  const size_t stage = (size_t)(Cs / 8) * kPlane, w = 1024 + conv_wbytes(NP, a.kp);
+  const int per_sm = w + 2 * stage <= 111u * 1024u ? 2 : 1;
+  a.ring = (int)std::min<size_t>(kMaxRing, ((per_sm == 2 ? 111u : 224u) * 1024u - w) / stage);
   const size_t smem = conv_smem_bytes(NP, a.kp, Cs, a.ring);
-  const int per_sm = std::max<int>(1, std::min<int>(2, (int)((227u * 1024u) / smem)));
   const int grid = std::min(a.ntiles, num_sms(dev) * per_sm);
   if (NP == 16) {
     if (mode == kFwdHidden) return launch_big(k_conv_tma<16, kFwdHidden>, grid, smem, s, m, a);
@@ -672,9 +756,8 @@ cudaError_t launch_conv(int dev, int mode, int NP, const __nv_bfloat16 *in, int 
 
 // Weight-gradient partials of one layer; returns the number of partials.
 cudaError_t launch_wgrad(int dev, const __nv_bfloat16 *a, int Cin, const __nv_bfloat16 *dz,
-                         int Cout, int nz, int nx, int ny, int taps,
-                         const __nv_bfloat16 *ones, float *part, int *err, cudaStream_t s,
-                         int *nchunk) {
+                         int Cout, int nz, int nx, int ny, int taps, float *part, int *err,
+                         cudaStream_t s, int *nchunk) {
   WgradArgs w;
   w.Csi = cstore(Cin);
   w.Cin = Cin;
@@ -684,20 +767,19 @@ cudaError_t launch_wgrad(int dev, const __nv_bfloat16 *a, int Cin, const __nv_bf
   w.nx = nx;
   w.ny = ny;
   w.taps = taps;
-  w.tiles_z = (nz + kTZ - 1) / kTZ;
-  w.tiles_x = (nx + kTX - 1) / kTX;
+  w.tiles_z = (nz + kWB - 1) / kWB;
+  w.tiles_x = (nx + kWB - 1) / kWB;
   w.ntiles = w.tiles_z * w.tiles_x * ny;
-  w.nmma = (taps * w.Csi + 8 + kTile - 1) / kTile;
-  w.ring = 5;
+  const size_t stage = wgrad_stage(w.Csi, w.Cso);
+  w.ring = (int)std::min<size_t>(kMaxRing, 200u * 1024u / stage);
   w.part = part;
   w.err = err;
-  CUtensorMap ma, md, mo;
-  if (!encode_act_map(&ma, a, w.Csi, nz, nx, ny, w.Csi / 8) ||
-      !encode_act_map(&md, dz, w.Cso, nz, nx, ny, w.Cso / 8) ||
-      !encode_act_map(&mo, ones, 8, kTZ, kTX, 1, 1))
+  CUtensorMap ma, md;
+  if (!encode_act_map(&ma, a, w.Csi, nz, nx, ny, kWZ, kWB + 2, true) ||
+      !encode_act_map(&md, dz, w.Cso, nz, nx, ny, kWB, kWB))
     return cudaErrorInvalidValue;
   const int NPO = r16(Cout);
-  const size_t smem = wgrad_smem_bytes(w.ring);
+  const size_t smem = 1024 + w.ring * stage;
   const int grid = std::min(w.ntiles, num_sms(dev));
   *nchunk = grid;
   cudaError_t e;
@@ -705,12 +787,12 @@ cudaError_t launch_wgrad(int dev, const __nv_bfloat16 *a, int Cin, const __nv_bf
     e = cudaFuncSetAttribute(k_wgrad_umma<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
     if (e != cudaSuccess) return e;
-    k_wgrad_umma<16><<<grid, kWsThreads, smem, s>>>(ma, md, mo, w);
+    k_wgrad_umma<16><<<grid, kWsThreads, smem, s>>>(ma, md, w);
   } else {
     e = cudaFuncSetAttribute(k_wgrad_umma<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
     if (e != cudaSuccess) return e;
-    k_wgrad_umma<32><<<grid, kWsThreads, smem, s>>>(ma, md, mo, w);
+    k_wgrad_umma<32><<<grid, kWsThreads, smem, s>>>(ma, md, w);
   }
   return cudaGetLastError();
 }
@@ -734,7 +816,6 @@ struct sw_cnn {
   float *out32 = nullptr, *in32 = nullptr, *tgt = nullptr, *part = nullptr;
   double *lpart = nullptr;
   int *err = nullptr;
-  __nv_bfloat16 *ones = nullptr;       // one 8-channel tile of BF16 ones (bias gradient)
 };
 
 namespace {
@@ -769,7 +850,8 @@ int ensure_images(sw_cnn *n, size_t npix) {
        ck(cudaMalloc(&n->out32, npix * sizeof(float))) &&
        ck(cudaMalloc(&n->in32, npix * n->ch[0] * sizeof(float))) &&
        ck(cudaMalloc(&n->tgt, npix * sizeof(float))) &&
-       ck(cudaMalloc(&n->part, (size_t)num_sms(n->ctx->device) * kWgradSlots * sizeof(float))) &&
+       ck(cudaMalloc(&n->part, (size_t)n->nl * num_sms(n->ctx->device) * part_floats(n->taps) *
+                               sizeof(float))) &&
        ck(cudaMalloc(&n->lpart, 1024 * sizeof(double)));
   if (!ok) {
     cudaGetLastError();
@@ -890,26 +972,30 @@ int gradient(sw_cnn *n, int nbatch, int nz, int nx, int ny, const float *in, con
             cudaSuccess ||
         (e = cudaMemcpyAsync(n->tgt, tin, npix * 4, cudaMemcpyHostToDevice, s)) != cudaSuccess)
       return cnn_fail(n, e, "cnn batch");
-    k_pack_input<<<nblk((long long)npix * cstore(n->ch[0])), 256, 0, s>>>(
-        n->in32, n->ch[0], cstore(n->ch[0]), (int)npix, n->a[0]);
+    k_pack_input<<<dim3(nblk(npix), cstore(n->ch[0]) / 8), 256, 0, s>>>(n->in32, n->ch[0], (int)npix,
+                                                                        n->a[0]);
     n->ctx->stats.launches_total++;
     if ((st = forward(n, nz, nx, ny))) return st;
     // d loss / d output (one channel), FP64 loss partials.
     int cur = 0;
     k_loss<<<lblocks, 256, 0, s>>>(n->out32, n->tgt, (int)npix, n->dz[cur], n->lpart);
     n->ctx->stats.launches_total++;
+    SumArgs sum;
+    sum.taps = T;
+    sum.g = n->g;
     for (int l = n->nl - 1; l >= 0; --l) {
       const int Cin = n->ch[l], Cout = n->ch[l + 1];
-      int nchunk = 0;
+      float *part = n->part + (size_t)l * num_sms(dev) * part_floats(T);
+      sum.part[l] = part;
+      sum.Cin[l] = Cin;
+      sum.Cout[l] = Cout;
+      sum.off[l] = n->woff[l];
       const uint64_t np = (uint64_t)npix;
       if ((e = timed_launch(n, np * (cstore(Cin) + cstore(Cout)) * 2, 2 * np * T * Cin * Cout, [&] {
-             return launch_wgrad(dev, n->a[l], Cin, n->dz[cur], Cout, nz, nx, ny, T, n->ones,
-                                 n->part, n->err, s, &nchunk);
+             return launch_wgrad(dev, n->a[l], Cin, n->dz[cur], Cout, nz, nx, ny, T, part, n->err,
+                                 s, &sum.nchunk);   // the same for every layer
            })) != cudaSuccess)
         return cnn_fail(n, e, "cnn wgrad");
-      k_wgrad_sum<<<T + 1, kMaxC * kMaxC, 0, s>>>(n->part, nchunk, Cout, Cin, T,
-                                                  n->g + n->woff[l]);
-      n->ctx->stats.launches_total++;
       if (l == 0) break;
       // Input gradient: mirrored taps, transposed weights, then ReLU' of
       // the layer input, into the other gradient buffer.
@@ -928,6 +1014,8 @@ int gradient(sw_cnn *n, int nbatch, int nz, int nx, int ny, const float *in, con
         return cnn_fail(n, e, "cnn dgrad");
       cur ^= 1;
     }
+    k_wgrad_sum<<<dim3(T + 1, kMaxC, n->nl), kSumW * kMaxC, 0, s>>>(sum);
+    n->ctx->stats.launches_total++;
     if ((e = cudaGetLastError()) != cudaSuccess) return cnn_fail(n, e, "cnn backward");
     if ((e = cudaMemcpyAsync(hp.data(), n->lpart, lblocks * sizeof(double),
                              cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
@@ -977,9 +1065,6 @@ int create_net(sw_ctx *c, int nlayers, const int *channels, uint64_t seed, int t
     ok = ck(cudaMalloc(&n->wf[l], (size_t)r16(Cout) * r16(taps * cstore(Cin)) * 2)) &&
          ck(cudaMalloc(&n->wb[l], (size_t)r16(Cin) * r16(taps * cstore(Cout)) * 2));
   }
-  const std::vector<unsigned short> one(8 * kTile, (unsigned short)0x3f80);   // BF16 1.0
-  ok = ok && ck(cudaMalloc(&n->ones, one.size() * 2)) &&
-       ck(cudaMemcpy(n->ones, one.data(), one.size() * 2, cudaMemcpyHostToDevice));
   ok = ok && ck(cudaMemcpy(n->w, h.data(), n->nw * 4, cudaMemcpyHostToDevice)) &&
        ck(cudaMemset(n->m, 0, n->nw * 4)) && ck(cudaMemset(n->v, 0, n->nw * 4)) &&
        ck(cudaMemset(n->err, 0, sizeof(int)));
@@ -1005,9 +1090,8 @@ int cnn_forward(sw_cnn *n, int nz, int nx, int ny, const float *in, float *out) 
   if ((e = cudaMemcpyAsync(n->in32, in, npix * n->ch[0] * 4, cudaMemcpyHostToDevice, s)) !=
       cudaSuccess)
     return cnn_fail(n, e, "cnn input");
-  k_pack_input<<<nblk((long long)npix * cstore(n->ch[0])), 256, 0, s>>>(n->in32, n->ch[0],
-                                                                     cstore(n->ch[0]), (int)npix,
-                                                                     n->a[0]);
+  k_pack_input<<<dim3(nblk(npix), cstore(n->ch[0]) / 8), 256, 0, s>>>(n->in32, n->ch[0], (int)npix,
+                                                                        n->a[0]);
   n->ctx->stats.launches_total++;
   if ((st = forward(n, nz, nx, ny))) return st;
   if ((e = cudaMemcpyAsync(out, n->out32, npix * 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
@@ -1065,7 +1149,6 @@ int sw_cnn_destroy(sw_cnn *n) {
   cudaStreamSynchronize(n->ctx->stream);
   free_images(n);
   cudaFree(n->w); cudaFree(n->g); cudaFree(n->m); cudaFree(n->v); cudaFree(n->err);
-  cudaFree(n->ones);
   for (auto p : n->wf) cudaFree(p);
   for (auto p : n->wb) cudaFree(p);
   delete n;
