@@ -282,13 +282,13 @@ __global__ void k_bv2u(BatchTables t, int s_off) {
 }
 
 // Snapshot save and RTM / LSRTM / AFWI imaging of step s for the 3D shots
-// of the pipelined kernel (the post-update part of t3_extras, which that
-// kernel leaves to this one): one thread per physical point, z fastest, on
+// of the pipelined kernel (which leaves them to k_bside3d): one thread per
+// physical point, z fastest, on
 // u2 of the step (the level the step kernel read, unchanged by it).  Per
 // element the operations of Propagator.f90:182-218 and Imaging.f90 as in
 // t3_extras.
-__global__ void k_bsnap3d(BatchTables t, int s_off) {
-  const int b = find_shot(t.snap_blocks, t.nshots, blockIdx.x);
+__device__ __forceinline__ void snap3d(const BatchTables &t, int s_off, int blk) {
+  const int b = find_shot(t.snap_blocks, t.nshots, blk);
   const ShotDev &S = t.shots[b];
   const int s = *t.counter + s_off;
   if (s >= S.nsteps) return;
@@ -333,7 +333,7 @@ __global__ void k_bsnap3d(BatchTables t, int s_off) {
     S.illum[q] = S.illum[q] + (wsn * wsn) * taper;
   };
   const int nb = t.snap_blocks[b + 1] - t.snap_blocks[b];
-  const long long first = (long long)(blockIdx.x - t.snap_blocks[b]) * blockDim.x + threadIdx.x;
+  const long long first = (long long)(blk - t.snap_blocks[b]) * blockDim.x + threadIdx.x;
   const long long stride = (long long)nb * blockDim.x;
   if ((g.nz & 3) == 0 && nphys < (1LL << 31)) {
     // 4 consecutive rows of a column per thread, 32-bit index arithmetic.
@@ -778,23 +778,50 @@ static cudaError_t launch_rho2d(const BatchTables &t, int s_off, int n_tiles, cu
   return cudaGetLastError();
 }
 
-// Sinc gather of one receiver in the loop order of Extraction_1trace_sinc_xy
-// (Extraction.f90:511-560) / _xyz (Extraction.f90:276-337).  H is the
-// half-width when known at compile time (lsinc = 7), else -1.
+// The 7 x 7 (x 7) gather of one receiver by a warp: every product first,
+// then the sum from tr, the same operations as the general loop below.
+template <int DIM>
+__device__ __forceinline__ float extract7(const Geom &g, const float *__restrict__ u2, int i0,
+                                          int j0, int k0, float v, const float *wz,
+                                          const float *wx, float tr, int lane) {
+  constexpr int NT = DIM == 2 ? 49 : 343, NC = (NT + 31) / 32;
+  float prod[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int tp = min(32 * c + lane, NT - 1);
+    const int ii = tp % 7, rest = tp / 7, jj = rest % 7, kq = rest / 7;
+    const float uv = u2[g.idx(i0 - 3 + ii, j0 - 3 + jj, DIM == 2 ? 1 : k0 - 3 + kq)];
+    prod[c] = ((v * uv) * wz[ii]) * wx[jj];
+    if (DIM == 3) prod[c] = prod[c] * wx[kq];   // the y weights are the x column
+  }
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    constexpr int last = NT - 32 * (NC - 1);
+#pragma unroll
+    for (int l = 0; l < (c == NC - 1 ? last : 32); ++l)
+      tr = tr + __shfl_sync(0xffffffffu, prod[c], l);
+  }
+  return tr;
+}
+
 // ---------------------------------------------------------------------------
 // Receiver extraction (Extraction.f90:71-135, 217-247, 276-337, 511-560):
 // one warp per receiver.  The lanes form the lsinc^2 (3D: lsinc^3) products
 // of a sinc gather 32 at a time, and lane 0 adds them to the trace sample
-// one by one in the reference's loop order (z fastest, then x, then y).
+// one by one in the reference's loop order (z fastest, then x, then y).  That
+// chain of adds, and the loads ahead of it, bound a warp: the 7-point gather
+// (ext_half 3) has all its loads in flight at once, and a launch takes the
+// samples of gridDim.y steps (s_off the first) together, as the steps' u2
+// stay in the rotating buffers for 4 steps.
 // ---------------------------------------------------------------------------
-__global__ void k_bextract(BatchTables t, int s_off) {
+__global__ void __launch_bounds__(128) k_bextract(BatchTables t, int s_off) {
   const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int ntot = t.rec_start[t.nshots];
   if (q >= ntot) return;   // uniform per warp
   const int b = find_shot(t.rec_start, t.nshots, q);
   const ShotDev &S = t.shots[b];
-  const int s = *t.counter + s_off;
+  const int s = *t.counter + s_off + blockIdx.y;
   if (s >= S.nsteps || S.ext_mode == 0) return;
   const int r = q - t.rec_start[b];
   const int it = S.tmin + s * S.tstep;
@@ -820,6 +847,12 @@ __global__ void k_bextract(BatchTables t, int s_off) {
   const int ntap = g.twoD ? ls * ls : ls * ls * ls;
   const float *wz = S.wz + (long long)r * ls, *wx = S.wx + (long long)r * ls;
   float tr = lane == 0 ? *trp : 0.f;
+  if (h == 3 && !S.ext_mirror) {
+    tr = g.twoD ? extract7<2>(g, u2, i0, j0, k0, v, wz, wx, tr, lane)
+                : extract7<3>(g, u2, i0, j0, k0, v, wz, wx, tr, lane);
+    if (lane == 0) *trp = tr;
+    return;
+  }
   for (int c0 = 0; c0 < ntap; c0 += 32) {
     const int tp = c0 + lane;
     float prod = 0.f;
@@ -1183,14 +1216,7 @@ __global__ void k_counter_add(int *counter, int add) {
 // 561-591); the step kernel adds a cell's terms in entry order.
 // sub = 1 forms the terms of the second step of a two-step launch (step
 // s_off - 1 + 1 of the counter) into the second block of inj_term.
-__global__ void k_bterms(BatchTables t, int s_off, int sub) {
-  // The next (step) kernel may start at once: it reads nothing this kernel
-  // or the previous step writes before its own wait, which returns only
-  // after this kernel completes - and this kernel completes only after the
-  // previous step kernel, which still reads the terms overwritten here.
-  pdl_launch_dependents();
-  pdl_wait();
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void form_term(const BatchTables &t, int s_off, int sub, int q) {
   if (q >= t.term_start[t.nshots]) return;
   const int b = find_shot(t.term_start, t.nshots, q);
   const ShotDev &S = t.shots[b];
@@ -1201,6 +1227,50 @@ __global__ void k_bterms(BatchTables t, int s_off, int sub) {
   const InjEntry E = S.inj_ent[k];
   const float tr = S.src_tr[(long long)E.tr * S.nt + (it - 1)];
   S.inj_term[(long long)sub * S.inj_nterm + k] = (((E.v2r * tr) * E.wz) * E.wx) * E.wy;
+}
+__global__ void k_bterms(BatchTables t, int s_off, int sub) {
+  // The next (step) kernel may start at once: it reads nothing this kernel
+  // or the previous step writes before its own wait, which returns only
+  // after this kernel completes - and this kernel completes only after the
+  // previous step kernel, which still reads the terms overwritten here.
+  pdl_launch_dependents();
+  pdl_wait();
+  form_term(t, s_off, sub, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// What follows the pipelined 3D step kernel of step s, in one launch: the
+// first n_term blocks form the injection terms of step s + 1, the next
+// n_edge blocks the absorbing edges of step s (edges3d), the rest its
+// snapshot saves and imaging.  The parts touch nothing in common: the edges
+// write u3 and read u2 and u1, the snapshots read u2.  Each is bound by
+// memory latency when it runs alone (240 x 440 x 440: z, x and y lines 33,
+// 15 and 12 us one after the other; 140 x 240 x 240: terms 7, snapshots 7 to
+// 27, lines 14, 10 and 8 us).
+constexpr int kSideThreads = 128;
+__global__ void __launch_bounds__(kSideThreads) k_bside3d(BatchTables t, int s_off, int n_term,
+                                                          int n_edge) {
+  int blk = blockIdx.x;
+  if (blk < n_term) {
+    form_term(t, s_off + 1, 0, blk * kSideThreads + threadIdx.x);
+    return;
+  }
+  blk -= n_term;
+  if (blk >= n_edge) {
+    snap3d(t, s_off, blk - n_edge);
+    return;
+  }
+  const int q = blk * kSideThreads + threadIdx.x;
+  if (q >= t.edge_start[t.nshots]) return;
+  const int b = find_shot(t.edge_start, t.nshots, q);
+  const ShotDev &S = t.shots[b];
+  const int s = *t.counter + s_off;
+  if (s < S.nsteps) edges3d(S, s, q - t.edge_start[b]);
+}
+
+cudaError_t launch_batch_extract(const BatchTables &t, int s_off, int nsteps, int n_rec,
+                                 cudaStream_t s) {
+  k_bextract<<<dim3((n_rec + 3) / 4, nsteps), 128, 0, s>>>(t, s_off);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_batch_step(const BatchTables &t, int s_off, int n_step_tiles, int n_rec,
@@ -1215,7 +1285,10 @@ cudaError_t launch_batch_step(const BatchTables &t, int s_off, int n_step_tiles,
     k_bextract<<<(n_rec + 3) / 4, 128, 0, s>>>(t, s_off);
     ++nl;
   }
-  if (n_term > 0) {
+  // The pipelined 3D kernel's terms: k_bside3d of the step before forms
+  // them, but for the first step of a chunk.
+  const bool side3d = has_3d && tile.stream3d == 2;
+  if (n_term > 0 && !(side3d && s_off > 0)) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((n_term + 255) / 256);
     cfg.blockDim = dim3(256);
@@ -1322,12 +1395,17 @@ cudaError_t launch_batch_step(const BatchTables &t, int s_off, int n_step_tiles,
     cudaError_t ec = record(ev_after);
     if (ec != cudaSuccess) return ec;
   }
-  // Snapshot saves and imaging of the pipelined 3D kernel's shots.
-  if (has_3d && tile.stream3d == 2 && tile.n_snap3d > 0) {
-    k_bsnap3d<<<tile.n_snap3d, 256, 0, s>>>(t, s_off);
-    ++nl;
+  if (side3d) {
+    const int nt = (n_term + kSideThreads - 1) / kSideThreads;
+    const int ne = (tile.n_edge + kSideThreads - 1) / kSideThreads;   // 0: lines by themselves
+    if (nt + ne + tile.n_snap3d > 0) {
+      k_bside3d<<<nt + ne + tile.n_snap3d, kSideThreads, 0, s>>>(t, s_off, nt, ne);
+      ++nl;
+    }
   }
-  if (tile.rigid) {
+  if (side3d && tile.n_edge > 0) {
+    // The edges of the step are done.
+  } else if (tile.rigid) {
     // Exact-adjoint mode: no absorbing boundary, the halo stays zero.
   } else if (!has_3d && (tile.stream2d == 2 || tile.stream2d == 3)) {
     // The pipelined 2D kernel applies the Higdon edges itself.
@@ -1339,7 +1417,7 @@ cudaError_t launch_batch_step(const BatchTables &t, int s_off, int n_step_tiles,
     k_bhiggx<<<(2 * n_hx + 127) / 128, 128, 0, s>>>(t, s_off);
     nl += 2;
   }
-  if (has_3d && n_hy > 0 && !tile.rigid) {
+  if (has_3d && n_hy > 0 && !tile.rigid && !(side3d && tile.n_edge > 0)) {
     k_bhiggy<<<(2 * n_hy + 127) / 128, 128, 0, s>>>(t, s_off);
     ++nl;
   }

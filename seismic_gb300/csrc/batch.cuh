@@ -224,7 +224,7 @@ struct StepTile {
   int nsm = 152;       // SMs of the device (persistent grids)
   int fused_edges = 0; // 2D: one launch for the z and x Higdon edges (set by the runner)
   int n_edge = 0;      // threads of that launch
-  int n_snap3d = 0;    // blocks of k_bsnap3d (pipelined 3D kernel with snapshots / imaging)
+  int n_snap3d = 0;    // blocks of k_bside3d for them (pipelined 3D kernel with snapshots / imaging)
   int rigid = 0;       // skip the Higdon boundary (exact-adjoint mode)
   int has_rho = 0;     // some shot runs the variable-density operator
   int rho2d = 0;       // every shot is 2D with a density: the one-pass k_brho2d
@@ -239,6 +239,24 @@ inline int edge_threads_2d(const Geom &g) {
   const int n1 = g.nmax1 - g.nmin1 + 1, n2 = g.nmax2 - g.nmin2 + 1;
   if (n1 < 16 || n2 < 16) return 0;
   return 128 + (2 * (n2 - 12) + 2 * (n1 - 8) + 31) / 32 * 32;
+}
+// Threads of a shot in the fused 3D edges (edges3d): z lines, x lines of the
+// inner rows, x lines of the 8
+// outer rows, y lines of the inner rows, y lines of the outer rows; each
+// part twice (near and far edge), rounded up to whole warps.
+__host__ __device__ inline int edge3d_part(const Geom &g, int part) {
+  const int n1 = g.nmax1 - g.nmin1 + 1, n2 = g.nmax2 - g.nmin2 + 1, n3 = g.nmax3 - g.nmin3 + 1;
+  const int n = part == 0   ? (n2 - 8) * (n3 - 8)
+                : part == 1 ? (n1 - 8) * (n3 - 8)
+                : part == 2 ? 8 * (n3 - 8)
+                : part == 3 ? (n1 - 8) * n2
+                            : 8 * n2;
+  return (n + 31) & ~31;
+}
+__host__ __device__ inline int edge_threads_3d(const Geom &g) {
+  int n = 0;
+  for (int part = 0; part < 5; ++part) n += 2 * edge3d_part(g, part);
+  return n;
 }
 
 // Number of fused-step CTAs a shot needs with this tile shape.
@@ -261,6 +279,13 @@ inline int step_ctas(const Geom &g, const StepTile &tile) {
   return ((n1 + 31) / 32) * ((n2 + 7) / 8) * n3;
 }
 
+// Receiver extraction of the nsteps steps from *counter + s_off, which have
+// all been taken (launch_batch_step with has_ext = 0).  A step's u2 is
+// overwritten by the 4th step after it (5 time levels): nsteps <= 4, before
+// that step; not with a free surface, which changes u2 at its own step.
+constexpr int kExtractSteps = 4;
+cudaError_t launch_batch_extract(const BatchTables &t, int s_off, int nsteps, int n_rec,
+                                 cudaStream_t s);
 // ev_before / ev_after (may be null) bracket the fused step kernel.
 cudaError_t launch_batch_step(const BatchTables &t, int s_off, int n_step_tiles, int n_rec,
                               int n_hz, int n_hx, int n_hy, int n_v2u, int has_ext, int has_3d,

@@ -16,10 +16,11 @@ namespace swave {
 //   u3(i) = -(g1 u3(i+d) + g2 u3(i+2d) + g3 u2(i) + g4 u2(i+d) + g5 u2(i+2d)
 //            + g6 u1(i) + g7 u1(i+d) + g8 u1(i+2d))
 // summed left to right, d the step towards the interior.
+// a and bq are the two u3 values inside the innermost output.
 __device__ __forceinline__ void higdon_half(const float *__restrict__ gc, long long cs,
                                             const float *__restrict__ u1,
                                             const float *__restrict__ u2, float *u3,
-                                            long long pstart, long long dst) {
+                                            long long pstart, long long dst, float a, float bq) {
   float c[8], U2[10], U1[10];
 #pragma unroll
   for (int q = 0; q < 8; ++q) c[q] = gc[q * cs];
@@ -29,7 +30,6 @@ __device__ __forceinline__ void higdon_half(const float *__restrict__ gc, long l
     U2[m] = u2[pm];
     U1[m] = u1[pm];
   }
-  float a = u3[pstart + dst], bq = u3[pstart + 2 * dst];
   float out[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
@@ -47,6 +47,34 @@ __device__ __forceinline__ void higdon_half(const float *__restrict__ gc, long l
   }
 #pragma unroll
   for (int k = 0; k < 8; ++k) u3[pstart - (long long)k * dst] = out[k];
+}
+__device__ __forceinline__ void higdon_half(const float *__restrict__ gc, long long cs,
+                                            const float *__restrict__ u1,
+                                            const float *__restrict__ u2, float *u3,
+                                            long long pstart, long long dst) {
+  higdon_half(gc, cs, u1, u2, u3, pstart, dst, u3[pstart + dst], u3[pstart + 2 * dst]);
+}
+
+// Output m (0: the innermost) of a half line, from the same operations,
+// without storing it.
+__device__ __forceinline__ float higdon_val(const float *__restrict__ gc, long long cs,
+                                            const float *__restrict__ u1,
+                                            const float *__restrict__ u2, long long pstart,
+                                            long long dst, float a, float bq, int m) {
+  for (int k = 0; k <= m; ++k) {
+    const long long p = pstart - (long long)k * dst;
+    float r = gc[0] * a;
+    r = r + gc[cs] * bq;
+    r = r + gc[2 * cs] * u2[p];
+    r = r + gc[3 * cs] * u2[p + dst];
+    r = r + gc[4 * cs] * u2[p + 2 * dst];
+    r = r + gc[5 * cs] * u1[p];
+    r = r + gc[6 * cs] * u1[p + dst];
+    r = r + gc[7 * cs] * u1[p + 2 * dst];
+    bq = a;
+    a = -r;
+  }
+  return a;
 }
 
 // One Higdon z half line (Boundary_3d, Boundary.f90:89-184) of column
@@ -155,6 +183,89 @@ __device__ __forceinline__ void higdon_xline(const ShotDev &S, int i, int k, boo
   const long long L = g.ld1;
   if (!right) higdon_half(S.gx + l, cs, u1, u2, u3, g.idx(i, g.nmin2 + 3, k), L);
   else higdon_half(S.gx + l + 8 * cs, cs, u1, u2, u3, g.idx(i, g.nmax2 - 3, k), -L);
+}
+
+// What the z lines, then the x lines leave in u3 at (i, j, k) (indices from
+// 0 over the compute domain; k not among the 4 outer planes), computed from
+// cells that no edge line writes: (i, j, k) itself, or up to two z lines and
+// an x line over them.
+__device__ __noinline__ float higdon_corner(const ShotDev &S, int i, int j, int k,
+                                            const float *u1, const float *u2, const float *u3) {
+  const Geom &g = S.g;
+  const int n1 = g.nmax1 - g.nmin1 + 1, n2 = g.nmax2 - g.nmin2 + 1, n3 = g.nmax3 - g.nmin3 + 1;
+  auto zed = [&](int jj) {
+    if (i >= 4 && i < n1 - 4) return u3[g.idx(g.nmin1 + i, g.nmin2 + jj, g.nmin3 + k)];
+    const bool bot = i >= 4;
+    const long long cs = (long long)n2 * n3, dst = bot ? -1 : 1;
+    const long long ps =
+        g.idx(bot ? g.nmax1 - 3 : g.nmin1 + 3, g.nmin2 + jj, g.nmin3 + k);
+    return higdon_val(S.gz + jj + (long long)n2 * k + (bot ? 8 * cs : 0), cs, u1, u2, ps, dst,
+                      u3[ps + dst], u3[ps + 2 * dst], 3 - (bot ? n1 - 1 - i : i));
+  };
+  if (j >= 4 && j < n2 - 4) return zed(j);
+  const bool right = j >= 4;
+  const long long cs = (long long)n1 * n3, dst = right ? -(long long)g.ld1 : g.ld1;
+  return higdon_val(S.gx + i + (long long)n1 * k + (right ? 8 * cs : 0), cs, u1, u2,
+                    g.idx(g.nmin1 + i, right ? g.nmax2 - 3 : g.nmin2 + 3, g.nmin3 + k), dst,
+                    zed(right ? n2 - 5 : 4), zed(right ? n2 - 6 : 5),
+                    3 - (right ? n2 - 1 - j : j));
+}
+
+// The 3D edges of a step in one launch, a thread per half line.  The
+// reference applies all z lines, then all x lines, then all y lines; a later
+// line overwrites the earlier ones' cells in the 4 outer columns or planes
+// and starts from two cells that an earlier one may have written.  So here a
+// z line of the outer 4 columns or planes, and an x line of the outer
+// planes, is left out (no later step reads the padding cells which only they
+// wrote), and a line that starts in a corner forms those two cells itself
+// (higdon_corner): the lines are independent.
+__device__ __forceinline__ void edges3d(const ShotDev &S, int s, int q) {
+  const Geom &g = S.g;
+  const int n1 = g.nmax1 - g.nmin1 + 1, n2 = g.nmax2 - g.nmin2 + 1, n3 = g.nmax3 - g.nmin3 + 1;
+  const float *u1 = S.f[(s + 2) % 5], *u2 = S.f[(s + 3) % 5];
+  float *u3 = S.f[(s + 4) % 5];
+  int part = 0, far = 0;
+  for (;; ++part) {
+    const int n = edge3d_part(g, part);
+    if (q < 2 * n) {
+      far = q >= n;
+      q -= far ? n : 0;
+      break;
+    }
+    q -= 2 * n;
+  }
+  if (part == 0) {
+    const int j = q % (n2 - 8) + 4, k = q / (n2 - 8) + 4;
+    if (k < n3 - 4) higdon_zline(S, g.nmin2 + j, g.nmin3 + k, far != 0, u1, u2, u3);
+    return;
+  }
+  // Row and, along x lines, plane (along y lines, column) of the line.
+  const int nr = part == 1 || part == 3 ? n1 - 8 : 8;
+  const int row = q % nr, o = q / nr;
+  const bool inner = part & 1;
+  const int i = inner || row >= 4 ? (inner ? row + 4 : n1 - 8 + row) : row;
+  if (part <= 2) {
+    const int k = o + 4;
+    if (k >= n3 - 4) return;
+    const long long cs = (long long)n1 * n3, dst = far ? -(long long)g.ld1 : g.ld1;
+    const long long ps = g.idx(g.nmin1 + i, far ? g.nmax2 - 3 : g.nmin2 + 3, g.nmin3 + k);
+    const float *gc = S.gx + i + (long long)n1 * k + (far ? 8 * cs : 0);
+    const float a = inner ? u3[ps + dst] : higdon_corner(S, i, far ? n2 - 5 : 4, k, u1, u2, u3);
+    const float b =
+        inner ? u3[ps + 2 * dst] : higdon_corner(S, i, far ? n2 - 6 : 5, k, u1, u2, u3);
+    higdon_half(gc, cs, u1, u2, u3, ps, dst, a, b);
+    return;
+  }
+  const int j = o;
+  if (j >= n2) return;
+  const long long P = g.plane();
+  const long long cs = (long long)n1 * n2, dst = far ? -P : P;
+  const long long ps = g.idx(g.nmin1 + i, g.nmin2 + j, far ? g.nmax3 - 3 : g.nmin3 + 3);
+  const float *gc = S.gy + i + (long long)n1 * j + (far ? 8 * cs : 0);
+  const bool plain = inner && j >= 4 && j < n2 - 4;
+  const float a = plain ? u3[ps + dst] : higdon_corner(S, i, j, far ? n3 - 5 : 4, u1, u2, u3);
+  const float b = plain ? u3[ps + 2 * dst] : higdon_corner(S, i, j, far ? n3 - 6 : 5, u1, u2, u3);
+  higdon_half(gc, cs, u1, u2, u3, ps, dst, a, b);
 }
 
 }  // namespace swave

@@ -217,9 +217,15 @@ extern "C" int sw_modeling_noalloc(const sw_genpar *g, const float *vel, const f
   t.counter = counter;
   t.err = err;
   // Time loop: step q reads s = *counter + q with the counter left at 0.
+  const bool late = ext.on && counts[1] > 0 && !tile.has_surf;
   for (int q = 0; q < nt; ++q) {
-    if (launch_batch_step(t, q, counts[0], counts[1], counts[2], counts[3], 0, 0, ext.on ? 1 : 0,
-                          0, 0, tile, s, nullptr, nullptr, nullptr) != cudaSuccess)
+    if (launch_batch_step(t, q, counts[0], counts[1], counts[2], counts[3], 0, 0,
+                          ext.on && !late ? 1 : 0, 0, 0, tile, s, nullptr, nullptr,
+                          nullptr) != cudaSuccess)
+      return SW_CUDA_ERR;
+    if (late && (q % kExtractSteps == kExtractSteps - 1 || q + 1 == nt) &&
+        launch_batch_extract(t, q - q % kExtractSteps, q % kExtractSteps + 1, counts[1], s) !=
+            cudaSuccess)
       return SW_CUDA_ERR;
   }
   if (nrec > 0 &&

@@ -165,6 +165,37 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
     }
     if (!fits) tile.stream2d = 1;
   }
+  if (!shots[0].d.g.twoD && tile.stream3d == 2 && tile.ty == StepTile{}.ty) {
+    // Planes per work unit of the pipelined 3D kernel (unless tuned): the
+    // CTAs take units in turn, so a launch lasts as long as the fullest CTA's
+    // units, each with about 3 planes' time to fill the pipeline.  32 planes
+    // gave 6 rounds for 5.2 units per CTA on 240 x 440 x 440 points (254 us
+    // per step) and 2 for 1.05 on 140 x 240 x 240 (77 us); 55 and 16 planes,
+    // chosen here, give 3 rounds and 2 shorter ones (228 and 64 us).  35
+    // planes and one round take 64 us there too, but longer where injection
+    // makes units unequal (a backward pass: 62.6 ms against 54.8 for the
+    // whole migration).
+    int nsm = 0, best = 0;
+    SW_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
+    long long bcost = 0;
+    for (int ty = 8; ty <= 128; ++ty) {
+      long long units = 0;
+      bool fits = true;   // at most 256 units in y (see below)
+      for (int b = 0; b < nb; ++b) {
+        const Geom g = make_geom(shots[b].d.g);
+        const int ny = (g.nmax3 - g.nmin3 + ty) / ty;
+        units += (long long)((g.nmax1 - g.nmin1 + 32) / 32) * ((g.nmax2 - g.nmin2 + 32) / 32) * ny;
+        fits = fits && ny <= 256;
+      }
+      if (!fits && ty < 128) continue;
+      const long long cost = (units + 2 * nsm - 1) / (2 * nsm) * (ty + 3);
+      if (best == 0 || cost < bcost) {
+        best = ty;
+        bcost = cost;
+      }
+    }
+    tile.ty = best;
+  }
   // The pipelined 3D kernel packs (shot, z tile, x tile, y unit) into 7/8/8/8
   // bits; larger batches or grids use the streaming kernel.
   if (!shots[0].d.g.twoD && tile.stream3d == 2) {
@@ -245,6 +276,18 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
   // The fused 2D edge kernel needs n1, n2 >= 16 in every shot.
   bool fused_edges = !has_3d && !tile.has_surf;
   for (int b = 0; b < nb && fused_edges; ++b) fused_edges = edge_threads_2d(G[b]) > 0;
+  // The 3D edges in one launch (edges3d) leave out padding cells next to the
+  // grid's edges that no receiver within the physical grid gathers from
+  // (half-widths are at most 7); the whole padded field of the last step, if
+  // asked for, still shows them.  Lines are 8 cells and start from 2 more.
+  bool edges3 = t3 && !tile.has_surf && !opt.rigid;
+  for (int b = 0; b < nb && edges3; ++b) {
+    const Geom &g = G[b];
+    const int w = std::min({1 - g.nmin1, g.nmax1 - g.nz, 1 - g.nmin2, g.nmax2 - g.nx,
+                            1 - g.nmin3, g.nmax3 - g.ny});
+    edges3 = w >= 8 && g.nmax1 - g.nmin1 >= 15 && g.nmax2 - g.nmin2 >= 15 &&
+             g.nmax3 - g.nmin3 >= 15 && !shots[b].io.final_u2_host;
+  }
   int max_steps = 0;
   for (int b = 0; b < nb; ++b) {
     const sw_prop_desc &d = shots[b].d;
@@ -396,18 +439,21 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
     hz[b + 1] = hz[b] + (int)(n2 * n3);
     hx[b + 1] = hx[b] + (int)(n1 * n3);
     hy[b + 1] = hy[b] + (g.twoD ? 0 : (int)(n1 * n2));
-    edge[b + 1] = edge[b] + (fused_edges ? edge_threads_2d(G[b]) : 0);
+    edge[b + 1] = edge[b] + (fused_edges ? edge_threads_2d(G[b])
+                             : edges3     ? edge_threads_3d(G[b])
+                                          : 0);
     // The pipelined 2D kernel adds injection terms computed per step by
     // k_bterms when a shot has many entries (receiver-side injection);
     // a few source entries are formed in the tile.
     term[b + 1] = term[b] + ((t2 || t3) && inj[b].on && inj[b].ent.size() >= kTermKernelMin
                                  ? (int)inj[b].ent.size() : 0);
     // The pipelined 3D kernel leaves a shot's snapshot saves and imaging to
-    // k_bsnap3d (one thread per physical point).
+    // k_bside3d (a thread per 4 physical points, or several: blocks for a few
+    // waves, as a step without a snapshot pays for starting them).
     S.inj_pre = term[b + 1] > term[b];
     snapb[b + 1] = snapb[b] + ((t3 && (S.extract_wave || S.imaging != 0))
                                    ? (int)std::min<long long>(
-                                         8192, ((long long)g.nz * g.nx * g.ny + 255) / 256)
+                                         2432, ((long long)g.nz * g.nx * g.ny + 511) / 512)
                                    : 0);
     v2b[b + 1] = v2b[b] + (((S.adj3d && !tile.stream3d) || S.rho_on)
                                ? (int)std::min<long long>(4096, (G[b].total() + 255) / 256)
@@ -636,7 +682,7 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
       uint64_t per_pt = 24;
       if (S.rho_on) per_pt = tile.rho2d ? 32 : (S.g.twoD ? 36 : 40);
       by += (uint64_t)S.npts * per_pt;
-      if (t3) continue;   // snapshots and imaging: k_bsnap3d
+      if (t3) continue;   // snapshots and imaging: k_bside3d
       const int it = S.tmin + sidx * S.tstep;
       if (it % S.snapi != 0) continue;
       const int cnt = S.tstep > 0 ? it / S.snapi - (S.tcnt - 1) / S.snapi
@@ -671,6 +717,10 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
     c->ev.resize(2 * chunk);
     for (size_t q = old; q < c->ev.size(); ++q) SW_CK(cudaEventCreate(&c->ev[q]));
   }
+  // Extraction after every 4th step for the 4 steps together: a warp's chain
+  // of adds takes 5 to 7 us whatever the number of receivers, a fifth of a
+  // small 2D step.
+  const bool late_ext = has_ext && n_rec > 0 && !tile.has_surf && !tile.fuse2;
   auto record_chunk = [&](int nsteps_here, bool with_events) -> int {
     int launched = 0;
     for (int q = 0; q < nsteps_here; q += stride) {
@@ -682,10 +732,16 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
       if (tile.fuse2)
         e = launch_batch_step2(t, q, n_tiles, n_rec, has_ext, tile, s, &nl, e0, e1, n_term);
       else
-        e = launch_batch_step(t, q, n_tiles, n_rec, n_hz, n_hx, n_hy, n_v2u, has_ext, has_3d,
-                              has_adj3d, tile, s, &nl, e0, e1, n_term);
+        e = launch_batch_step(t, q, n_tiles, n_rec, n_hz, n_hx, n_hy, n_v2u,
+                              has_ext && !late_ext, has_3d, has_adj3d, tile, s, &nl, e0, e1,
+                              n_term);
       if (e != cudaSuccess) return -1;
       launched += nl;
+      if (late_ext && (q % kExtractSteps == kExtractSteps - 1 || q + 1 == nsteps_here)) {
+        const int q0 = q - q % kExtractSteps;
+        if ((e = launch_batch_extract(t, q0, q + 1 - q0, n_rec, s)) != cudaSuccess) return -1;
+        ++launched;
+      }
     }
     if ((e = launch_counter_add(counter, nsteps_here, s)) != cudaSuccess) return -1;
     return launched + 1;

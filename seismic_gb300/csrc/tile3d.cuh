@@ -344,7 +344,7 @@ __device__ __forceinline__ void tile3d_persistent(const BatchTables &t, int s_of
           for (int r = 0; r < 4; ++r)
             if (i0 + r <= g.nmax1) u3[off + r] = o[r];
         }
-        // Snapshot saves and imaging of this step: k_bsnap3d, after the
+        // Snapshot saves and imaging of this step: k_bside3d, after the
         // launch.
       }
       __syncthreads();   // the stage is free for plane p + S
