@@ -454,30 +454,31 @@ __global__ void k_brho_grad(BatchTables t, int s_off) {
 // The 2D variable-density step in one pass (FDderivatives.f90:601-657 and
 // the time update): each block owns a tile of 64 (z) x 32 (x) outputs.  At
 // its start it issues asynchronous 16-byte copies (cp.async, zero-filled
-// outside the padded array) of every input into shared memory: u2 with an
-// 8-cell halo (80 x 48), delp with a 4-cell halo (72 x 40), and the tile's
-// v, rho, u1, u0 and u_1 (64 x 32 each).  It then forms the staggered
-// gradients the tile's divergence reads - sz on rows z0-4..z0+67 of the
-// tile's columns, sx on columns x0-4..x0+35 of its rows - with the
-// operations and padding-cell rules of k_brho_grad, and finally the
-// divergence times v^2*rho and the rest of the point update (step_tail).
+// outside the padded array) into shared memory of what the gradients read:
+// u2 with an 8-cell halo (80 x 48) and delp with a 4-cell halo (72 x 40).
+// It then forms the staggered gradients the tile's divergence reads - sz on
+// rows z0-4..z0+67 of the tile's columns, sx on columns x0-4..x0+35 of its
+// rows - with the operations and padding-cell rules of k_brho_grad, and
+// finally the divergence times v^2*rho and the rest of the point update
+// (step_tail), whose v, rho, u1, u0 and u_1 it reads straight into
+// registers.  Tiles at the boundary come first in the grid and, with `edges`,
+// end with the Higdon lines of their columns and rows.
 // sz and sx never go through HBM: 32 bytes per point (u2, delp, v, rho, u1,
 // u0, u_1 read, u3 written) instead of the two passes' 52.
 // ---------------------------------------------------------------------------
 constexpr int R2_Z = 64, R2_X = 32;
 constexpr int R2_UZ = R2_Z + 16, R2_UX = R2_X + 16;   // staged u2: rows z0-8.., columns x0-8..
 constexpr int R2_GZ = R2_Z + 8, R2_GX = R2_X + 8;     // delp and sz rows z0-4.., sx columns x0-4..
-constexpr int R2_CORE = R2_Z * R2_X;
 // Shared-memory layout in floats, every array [column][row].
 constexpr int R2_SU = 0;                                // u2, R2_UX x R2_UZ
 constexpr int R2_SDP = R2_SU + R2_UX * R2_UZ;           // delp, R2_GX x R2_GZ
-constexpr int R2_SC = R2_SDP + R2_GX * R2_GZ;           // v, rho, u1, u0, u_1: 5 x R2_CORE
-constexpr int R2_SSZ = R2_SC + 5 * R2_CORE;             // sz, R2_X x R2_GZ
+constexpr int R2_SSZ = R2_SDP + R2_GX * R2_GZ;          // sz, R2_X x R2_GZ
 constexpr int R2_SSX = R2_SSZ + R2_X * R2_GZ;           // sx, R2_GX x R2_Z
 constexpr int R2_FLOATS = R2_SSX + R2_GX * R2_Z;
-constexpr size_t R2_SMEM = sizeof(float) * R2_FLOATS;   // 87 296 bytes: two blocks per SM
+constexpr size_t R2_SMEM = sizeof(float) * R2_FLOATS;   // 46 336 bytes
 // 16-byte chunks of the staged arrays.
-constexpr int R2_QU = R2_UX * (R2_UZ / 4), R2_QD = R2_GX * (R2_GZ / 4), R2_QC = R2_X * (R2_Z / 4);
+constexpr int R2_QU = R2_UX * (R2_UZ / 4), R2_QD = R2_GX * (R2_GZ / 4);
+constexpr int R2_PER_SM = 3;   // resident blocks
 
 // 16-byte asynchronous global -> shared copy; with in false nothing is read
 // and the destination is zero-filled.
@@ -512,9 +513,9 @@ __device__ __forceinline__ void lds4_to(float *r, const float *p) {
   r[3] = v.w;
 }
 
-__global__ void __launch_bounds__(256, 2) k_brho2d(BatchTables t, int s_off) {
+__global__ void __launch_bounds__(256, R2_PER_SM) k_brho2d(BatchTables t, int s_off, int edges) {
   extern __shared__ __align__(16) float r2s[];
-  float *su = r2s + R2_SU, *sdp = r2s + R2_SDP, *sc = r2s + R2_SC;
+  float *su = r2s + R2_SU, *sdp = r2s + R2_SDP;
   float *ssz = r2s + R2_SSZ, *ssx = r2s + R2_SSX;
   const int b = find_shot(t.step_tiles, t.nshots, blockIdx.x);
   const ShotDev &S = t.shots[b];
@@ -523,17 +524,34 @@ __global__ void __launch_bounds__(256, 2) k_brho2d(BatchTables t, int s_off) {
   const Geom &g = S.g;
   const int nmin1 = g.nmin1, nmax1 = g.nmax1, nmin2 = g.nmin2, nmax2 = g.nmax2;
   const int lo1 = g.lo1, lo2 = g.lo2, ld = g.ld1, n2p = g.n2p;
-  const int ntz = (nmax1 - nmin1 + R2_Z) / R2_Z;
-  const int local = blockIdx.x - t.step_tiles[b];
-  const int z0 = nmin1 + (local % ntz) * R2_Z, x0 = nmin2 + (local / ntz) * R2_X;
+  const int n1 = nmax1 - nmin1 + 1, n2 = nmax2 - nmin2 + 1;
+  const int o1 = r2_origin(n1, R2_Z, 4), o2 = r2_origin(n2, R2_X, 1);
+  const int ntz = (n1 + o1 + R2_Z - 1) / R2_Z;
+  const int ntx = (n2 + o2 + R2_X - 1) / R2_X;
+  int local = blockIdx.x - t.step_tiles[b], tzi, txi;
+  if (ntz < 3 || ntx < 3) {
+    tzi = local % ntz;
+    txi = local / ntz;
+  } else if (local < 2 * ntx) {
+    tzi = local < ntx ? 0 : ntz - 1;
+    txi = local < ntx ? local : local - ntx;
+  } else if ((local -= 2 * ntx) < 2 * (ntz - 2)) {
+    txi = local < ntz - 2 ? 0 : ntx - 1;
+    tzi = 1 + (local < ntz - 2 ? local : local - (ntz - 2));
+  } else {
+    local -= 2 * (ntz - 2);
+    tzi = 1 + local % (ntz - 2);
+    txi = 1 + local / (ntz - 2);
+  }
+  const int z0 = nmin1 - o1 + tzi * R2_Z, x0 = nmin2 - o2 + txi * R2_X;
   const int tid = threadIdx.x;
-  const float *__restrict__ u2 = S.f[(s + 3) % 5];
-  float *__restrict__ u3 = S.f[(s + 4) % 5];
+  const float *u2 = S.f[(s + 3) % 5];
+  float *u3 = S.f[(s + 4) % 5];
   // 32-bit offsets in the padded array (fewer than 2^31 points per shot,
   // checked when the batch is set up).
   auto off = [&](int i, int j) { return (i - lo1) + ld * (j - lo2); };
-  // Every chunk starts 4k rows after the padded array's first row (z0 - lo1
-  // = 64 t + 4), so a chunk lies wholly inside a column's ld1 rows or wholly
+  // Every chunk starts a multiple of 4 rows from the padded array's first row
+  // (z0 - lo1 = 64 t + 4 - o1), so a chunk lies wholly inside a column's ld1 rows or wholly
   // outside them; the arrays are 256-byte aligned and ld1 is a multiple of
   // 32, so every source address is 16-byte aligned.  Cells beyond the
   // padded array (zero-filled, or rows n1p..ld1-1 of a column) feed no value
@@ -551,22 +569,7 @@ __global__ void __launch_bounds__(256, 2) k_brho2d(BatchTables t, int s_off) {
     const int cc = q / (R2_GZ / 4), k = q - cc * (R2_GZ / 4);
     stage(sdp + cc * R2_GZ + 4 * k, S.delp, z0 - 4 + 4 * k, x0 - 4 + cc);
   }
-  cp_async_commit();   // group 1: what the gradients read
-  {
-    // v, rho, then u1, u0, u_1 (levels s+2, s+1, s of the 5-level ring):
-    // two chunks of each per thread.
-    static_assert(R2_QC == 2 * 256, "core chunks per thread");
-#pragma unroll
-    for (int a = 0; a < 5; ++a) {
-      const float *src = a == 0 ? S.vel : a == 1 ? S.rho : S.f[(s + 4 - a) % 5];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int q = tid + 256 * h, cc = q >> 4, k = q & 15;
-        stage(sc + a * R2_CORE + cc * R2_Z + 4 * k, src, z0 + 4 * k, x0 + cc);
-      }
-    }
-  }
-  cp_async_commit();   // group 2: the point update's inputs
+  cp_async_commit();
   // The shot's scalars, loaded while the copies are in flight.
   const Coefs &cf = S.cr;
   const float c1z = cf.c1z, c2z = cf.c2z, c3z = cf.c3z, c4z = cf.c4z;
@@ -581,7 +584,7 @@ __global__ void __launch_bounds__(256, 2) k_brho2d(BatchTables t, int s_off) {
   // 960-982), done below on four rows at once.
   const bool heavy = inj_tile || (snapstep && (S.imaging != 0 || S.extract_wave));
   const float k12 = S.k12, div11 = S.div11;
-  cp_async_wait<1>();
+  cp_async_wait<0>();
   __syncthreads();
   // sz at rows z0-4+rr..+3 of column x0+cc, four rows per item: the
   // 8th-order difference times delp inside the compute domain, the
@@ -590,7 +593,7 @@ __global__ void __launch_bounds__(256, 2) k_brho2d(BatchTables t, int s_off) {
   // writes) and off the compute columns.  delp at (i, j) is
   // sdp[(j - x0 + 4) * R2_GZ + i - z0 + 4]; a face row or column that a
   // padding cell of the tile needs lies inside the staged 72 x 40 block
-  // (z0 >= nmin1, x0 >= nmin2).
+  // (a tile within 3 rows or columns of a face, or across it, stages it).
   // A tile whose gradient cells all lie inside the compute domain (most of
   // them) takes the 8th-order difference everywhere, without the per-cell
   // domain and padding tests.
@@ -636,7 +639,7 @@ __global__ void __launch_bounds__(256, 2) k_brho2d(BatchTables t, int s_off) {
       const int cc = q / (R2_GZ / 4), rr = 4 * (q - cc * (R2_GZ / 4));
       const int i0 = z0 - 4 + rr, j = x0 + cc;
       float v[4] = {0.f, 0.f, 0.f, 0.f};
-      if (j <= nmax2) {
+      if (j <= nmax2 && j >= nmin2) {
         // u2 at rows i0-3..i0+7 of column j: staged rows rr+1..rr+11.
         float U[12], D[4];
         const float *col = su + (cc + 8) * R2_UZ + rr;
@@ -692,8 +695,9 @@ __global__ void __launch_bounds__(256, 2) k_brho2d(BatchTables t, int s_off) {
       *reinterpret_cast<float4 *>(ssx + cc * R2_Z + rr) = make_float4(v[0], v[1], v[2], v[3]);
     }
   }
-  cp_async_wait<0>();
   __syncthreads();
+  const float *const pv = S.vel, *const pr = S.rho, *const f1 = S.f[(s + 2) % 5],
+              *const f0 = S.f[(s + 1) % 5], *const fm = S.f[s % 5];
   // Divergence times v^2*rho (FDderivatives.f90:642-655) and the point
   // update, four rows per item: lanes 0-15 of a warp take the 16 row
   // groups of one column, lanes 16-31 those of the next.
@@ -701,7 +705,14 @@ __global__ void __launch_bounds__(256, 2) k_brho2d(BatchTables t, int s_off) {
 #pragma unroll 1
   for (int h = 0; h < 2; ++h) {
     const int cc = (tid >> 4) + 16 * h, j = x0 + cc, i0 = z0 + rr;
-    if (j > nmax2 || i0 > nmax1) continue;
+    if (j > nmax2 || i0 > nmax1 || j < nmin2 || i0 < nmin1) continue;
+    const int p0 = off(i0, j);
+    float VV[4], RH[4], A1[4], A0[4], AM[4], U2[4];
+    lds4_to(VV, pv + p0);
+    lds4_to(RH, pr + p0);
+    lds4_to(A1, f1 + p0);
+    lds4_to(A0, f0 + p0);
+    lds4_to(AM, fm + p0);
     // sz at rows i0-4..i0+7: Z[m] is row i0-4+m.
     float Z[12];
     const float *zc = ssz + cc * R2_GZ + rr;
@@ -712,13 +723,6 @@ __global__ void __launch_bounds__(256, 2) k_brho2d(BatchTables t, int s_off) {
     float X[8][4];
 #pragma unroll
     for (int m = 0; m < 8; ++m) lds4_to(X[m], ssx + (cc + m) * R2_Z + rr);
-    float VV[4], RH[4], A1[4], A0[4], AM[4], U2[4];
-    const float *cv = sc + cc * R2_Z + rr;
-    lds4_to(VV, cv);
-    lds4_to(RH, cv + R2_CORE);
-    lds4_to(A1, cv + 2 * R2_CORE);
-    lds4_to(A0, cv + 3 * R2_CORE);
-    lds4_to(AM, cv + 4 * R2_CORE);
     lds4_to(U2, su + (cc + 8) * R2_UZ + rr + 8);
     float sv[4];
 #pragma unroll
@@ -734,7 +738,6 @@ __global__ void __launch_bounds__(256, 2) k_brho2d(BatchTables t, int s_off) {
       const float vr = (VV[e] * VV[e]) * RH[e];
       sv[e] = vr * (tx + tz);
     }
-    const int p0 = off(i0, j);
     if (heavy) {
 #pragma unroll
       for (int e = 0; e < 4; ++e)
@@ -761,9 +764,32 @@ __global__ void __launch_bounds__(256, 2) k_brho2d(BatchTables t, int s_off) {
         if (i0 + e <= nmax1) u3[p0 + e] = o[e];
     }
   }
+  if (!edges) return;
+  // Higdon edges (Boundary.f90:89-184): z lines, then x lines.  A line's
+  // cells of u3 lie in this tile (r2_origin).
+  const bool top = tzi == 0, bottom = tzi == ntz - 1, left = txi == 0, right = txi == ntx - 1;
+  if (!(top || bottom || left || right)) return;
+  __syncthreads();
+  if (tid < 2 * R2_X) {
+    const bool bot = tid >= R2_X;
+    const int j = x0 + (tid & (R2_X - 1));
+    if ((bot ? bottom : top) && j >= nmin2 && j <= nmax2)
+      higdon_half(S.gz + (j - nmin2) + (bot ? 8 * n2 : 0), n2, f1, u2, u3,
+                  off(bot ? nmax1 - 3 : nmin1 + 3, j), bot ? -1 : 1);
+  }
+  if (!(left || right)) return;
+  __syncthreads();
+  if (tid < 2 * R2_Z) {
+    const bool rgt = tid >= R2_Z;
+    const int i = z0 + (tid & (R2_Z - 1));
+    if ((rgt ? right : left) && i >= nmin1 && i <= nmax1)
+      higdon_half(S.gx + (i - nmin1) + (rgt ? 8 * n1 : 0), n1, f1, u2, u3,
+                  off(i, rgt ? nmax2 - 3 : nmin2 + 3), rgt ? -ld : ld);
+  }
 }
 
-static cudaError_t launch_rho2d(const BatchTables &t, int s_off, int n_tiles, cudaStream_t s) {
+static cudaError_t launch_rho2d(const BatchTables &t, int s_off, int n_tiles, int edges,
+                                cudaStream_t s) {
   // The shared-memory opt-in is a per-device function attribute.
   static unsigned long long attr_set = 0;
   int dev = 0;
@@ -774,7 +800,7 @@ static cudaError_t launch_rho2d(const BatchTables &t, int s_off, int n_tiles, cu
     if (e != cudaSuccess) return e;
     if (dev < 64) attr_set |= 1ull << dev;
   }
-  k_brho2d<<<n_tiles, 256, R2_SMEM, s>>>(t, s_off);
+  k_brho2d<<<n_tiles, 256, R2_SMEM, s>>>(t, s_off, edges);
   return cudaGetLastError();
 }
 
@@ -1384,7 +1410,7 @@ cudaError_t launch_batch_step(const BatchTables &t, int s_off, int n_step_tiles,
     else if (tile.tz == 32) launch_stream2d<32>(t, s_off, n_step_tiles, tile, hf, ha, s, &nl);
     else launch_stream2d<64>(t, s_off, n_step_tiles, tile, hf, ha, s, &nl);
   } else if (tile.rho2d) {
-    cudaError_t e = launch_rho2d(t, s_off, n_step_tiles, s);
+    cudaError_t e = launch_rho2d(t, s_off, n_step_tiles, tile.rho_edges, s);
     if (e != cudaSuccess) return e;
     ++nl;
   } else {
@@ -1409,6 +1435,8 @@ cudaError_t launch_batch_step(const BatchTables &t, int s_off, int n_step_tiles,
     // Exact-adjoint mode: no absorbing boundary, the halo stays zero.
   } else if (!has_3d && (tile.stream2d == 2 || tile.stream2d == 3)) {
     // The pipelined 2D kernel applies the Higdon edges itself.
+  } else if (tile.rho2d && tile.rho_edges) {
+    // k_brho2d too.
   } else if (!has_3d && tile.fused_edges) {
     k_bedges2d<<<(tile.n_edge + 127) / 128, 128, 0, s>>>(t, s_off);
     ++nl;

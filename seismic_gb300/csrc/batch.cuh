@@ -116,6 +116,16 @@ inline bool t2_origin(int n1, int n2, int *off1, int *off2, int *ntz, int *ntx) 
   return true;
 }
 
+// Cells that k_brho2d's first tile along an axis of n cells starts before the
+// compute domain (tiles of T, a multiple of step): the fewest that leave at
+// least 6 cells to the last tile, so that what an edge line writes or starts
+// from lies in one tile.
+__host__ __device__ inline int r2_origin(int n, int T, int step) {
+  for (int o = 0; o <= T - 8; o += step)
+    if ((n + o - 1) % T >= 5) return o;
+  return 0;   // n below 6
+}
+
 // Largest batch the pipelined 2D kernel accepts (its shot table is shared).
 constexpr int T2_MAX_SHOTS = 64;
 // Largest batch of the two-step 2D kernel (tile2d2.cuh).
@@ -227,6 +237,7 @@ struct StepTile {
   int n_snap3d = 0;    // blocks of k_bside3d for them (pipelined 3D kernel with snapshots / imaging)
   int rigid = 0;       // skip the Higdon boundary (exact-adjoint mode)
   int has_rho = 0;     // some shot runs the variable-density operator
+  int rho_edges = 0;   // k_brho2d applies the Higdon edges itself
   int rho2d = 0;       // every shot is 2D with a density: the one-pass k_brho2d
   int has_surf = 0;    // some shot has a free surface (point tiles, k_bfree)
   int fuse2 = 0;       // 2D tiles: two time steps per launch (tile2d2.cuh)
@@ -262,7 +273,8 @@ __host__ __device__ inline int edge_threads_3d(const Geom &g) {
 // Number of fused-step CTAs a shot needs with this tile shape.
 inline int step_ctas(const Geom &g, const StepTile &tile) {
   const int n1 = g.nmax1 - g.nmin1 + 1, n2 = g.nmax2 - g.nmin2 + 1, n3 = g.nmax3 - g.nmin3 + 1;
-  if (g.twoD && tile.rho2d) return ((n1 + 63) / 64) * ((n2 + 31) / 32);
+  if (g.twoD && tile.rho2d)
+    return ((n1 + r2_origin(n1, 64, 4) + 63) / 64) * ((n2 + r2_origin(n2, 32, 1) + 31) / 32);
   if (g.twoD && tile.fuse2) {
     int o1, o2, nz, nx;
     return tf_origin(n1, n2, &o1, &o2, &nz, &nx) ? nz * nx : 0;

@@ -645,6 +645,7 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
   tile.has_fwd2d = tile.has_adj2d = tile.has_fwd3d = tile.has_adj3d = 0;
   tile.fused_edges = fused_edges ? 1 : 0;
   tile.rigid = opt.rigid ? 1 : 0;
+  tile.rho_edges = tile.rho2d && fused_edges && !opt.rigid;
   tile.n_edge = edge[nb];
 
   for (auto &S : hs) {
