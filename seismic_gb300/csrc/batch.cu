@@ -514,13 +514,17 @@ __device__ __forceinline__ void lds4_to(float *r, const float *p) {
 }
 
 __global__ void __launch_bounds__(256, R2_PER_SM) k_brho2d(BatchTables t, int s_off, int edges) {
+  pdl_launch_dependents();
   extern __shared__ __align__(16) float r2s[];
   float *su = r2s + R2_SU, *sdp = r2s + R2_SDP;
   float *ssz = r2s + R2_SSZ, *ssx = r2s + R2_SSX;
   const int b = find_shot(t.step_tiles, t.nshots, blockIdx.x);
   const ShotDev &S = t.shots[b];
   const int s = *t.counter + s_off;
-  if (s >= S.nsteps) return;   // the whole block
+  if (s >= S.nsteps) {   // the whole block
+    pdl_wait();
+    return;
+  }
   const Geom &g = S.g;
   const int nmin1 = g.nmin1, nmax1 = g.nmax1, nmin2 = g.nmin2, nmax2 = g.nmax2;
   const int lo1 = g.lo1, lo2 = g.lo2, ld = g.ld1, n2p = g.n2p;
@@ -561,13 +565,14 @@ __global__ void __launch_bounds__(256, R2_PER_SM) k_brho2d(BatchTables t, int s_
     const bool in = i0 >= lo1 && i0 < lo1 + ld && j >= lo2 && j < lo2 + n2p;
     cp_async16(dst, in ? src + off(i0, j) : src, in);
   };
-  for (int q = tid; q < R2_QU; q += 256) {
-    const int cc = q / (R2_UZ / 4), k = q - cc * (R2_UZ / 4);
-    stage(su + cc * R2_UZ + 4 * k, u2, z0 - 8 + 4 * k, x0 - 8 + cc);
-  }
   for (int q = tid; q < R2_QD; q += 256) {
     const int cc = q / (R2_GZ / 4), k = q - cc * (R2_GZ / 4);
     stage(sdp + cc * R2_GZ + 4 * k, S.delp, z0 - 4 + 4 * k, x0 - 4 + cc);
+  }
+  pdl_wait();   // the steps before
+  for (int q = tid; q < R2_QU; q += 256) {
+    const int cc = q / (R2_UZ / 4), k = q - cc * (R2_UZ / 4);
+    stage(su + cc * R2_UZ + 4 * k, u2, z0 - 8 + 4 * k, x0 - 8 + cc);
   }
   cp_async_commit();
   // The shot's scalars, loaded while the copies are in flight.
@@ -800,8 +805,21 @@ static cudaError_t launch_rho2d(const BatchTables &t, int s_off, int n_tiles, in
     if (e != cudaSuccess) return e;
     if (dev < 64) attr_set |= 1ull << dev;
   }
-  k_brho2d<<<n_tiles, 256, R2_SMEM, s>>>(t, s_off, edges);
-  return cudaGetLastError();
+  // Programmatic dependent launch within a chunk: the blocks start (tables,
+  // delp into shared memory) as the previous kernel's retire and wait in the
+  // kernel.  Not as the first of a chunk: what a block reads before its wait,
+  // the step counter and the tables, was in place before the chunk.
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(n_tiles);
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = R2_SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = s_off > 0 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k_brho2d, t, s_off, edges);
 }
 
 // The 7 x 7 (x 7) gather of one receiver by a warp: every product first,
