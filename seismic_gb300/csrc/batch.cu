@@ -466,7 +466,7 @@ __global__ void k_brho_grad(BatchTables t, int s_off) {
 // sz and sx never go through HBM: 32 bytes per point (u2, delp, v, rho, u1,
 // u0, u_1 read, u3 written) instead of the two passes' 52.
 // ---------------------------------------------------------------------------
-constexpr int R2_Z = 64, R2_X = 32;
+constexpr int R2_Z = 32, R2_X = 32, R2_G = R2_Z / 4;   // R2_G: row groups
 constexpr int R2_UZ = R2_Z + 16, R2_UX = R2_X + 16;   // staged u2: rows z0-8.., columns x0-8..
 constexpr int R2_GZ = R2_Z + 8, R2_GX = R2_X + 8;     // delp and sz rows z0-4.., sx columns x0-4..
 // Shared-memory layout in floats, every array [column][row].
@@ -478,7 +478,7 @@ constexpr int R2_FLOATS = R2_SSX + R2_GX * R2_Z;
 constexpr size_t R2_SMEM = sizeof(float) * R2_FLOATS;   // 46 336 bytes
 // 16-byte chunks of the staged arrays.
 constexpr int R2_QU = R2_UX * (R2_UZ / 4), R2_QD = R2_GX * (R2_GZ / 4);
-constexpr int R2_PER_SM = 3;   // resident blocks
+constexpr int R2_PER_SM = 4;   // resident blocks
 
 // 16-byte asynchronous global -> shared copy; with in false nothing is read
 // and the destination is zero-filled.
@@ -624,7 +624,7 @@ __global__ void __launch_bounds__(256, R2_PER_SM) k_brho2d(BatchTables t, int s_
       *reinterpret_cast<float4 *>(ssz + cc * R2_GZ + rr) = make_float4(v[0], v[1], v[2], v[3]);
     }
     for (int q = tid; q < R2_GX * (R2_Z / 4); q += 256) {
-      const int cc = q >> 4, rr = 4 * (q & 15);
+      const int cc = q / R2_G, rr = 4 * (q % R2_G);
       float V[8][4], D[4], v[4];
 #pragma unroll
       for (int m = 0; m < 8; ++m) lds4_to(V[m], su + (cc + 1 + m) * R2_UZ + rr + 8);
@@ -672,7 +672,7 @@ __global__ void __launch_bounds__(256, R2_PER_SM) k_brho2d(BatchTables t, int s_
     }
     // sx at rows z0+rr..+3 of column x0-4+cc, by the same rules along x.
     for (int q = tid; q < R2_GX * (R2_Z / 4); q += 256) {
-      const int cc = q >> 4, rr = 4 * (q & 15);
+      const int cc = q / R2_G, rr = 4 * (q % R2_G);
       const int i0 = z0 + rr, j = x0 - 4 + cc;
       float v[4] = {0.f, 0.f, 0.f, 0.f};
       const bool jin = j >= nmin2 && j <= nmax2;
@@ -706,10 +706,10 @@ __global__ void __launch_bounds__(256, R2_PER_SM) k_brho2d(BatchTables t, int s_
   // Divergence times v^2*rho (FDderivatives.f90:642-655) and the point
   // update, four rows per item: lanes 0-15 of a warp take the 16 row
   // groups of one column, lanes 16-31 those of the next.
-  const int rr = 4 * (tid & 15);
+  const int rr = 4 * (tid % R2_G);
 #pragma unroll 1
-  for (int h = 0; h < 2; ++h) {
-    const int cc = (tid >> 4) + 16 * h, j = x0 + cc, i0 = z0 + rr;
+  for (int h = 0; h < R2_X * R2_G / 256; ++h) {
+    const int cc = tid / R2_G + 256 / R2_G * h, j = x0 + cc, i0 = z0 + rr;
     if (j > nmax2 || i0 > nmax1 || j < nmin2 || i0 < nmin1) continue;
     const int p0 = off(i0, j);
     float VV[4], RH[4], A1[4], A0[4], AM[4], U2[4];

@@ -274,7 +274,7 @@ __host__ __device__ inline int edge_threads_3d(const Geom &g) {
 inline int step_ctas(const Geom &g, const StepTile &tile) {
   const int n1 = g.nmax1 - g.nmin1 + 1, n2 = g.nmax2 - g.nmin2 + 1, n3 = g.nmax3 - g.nmin3 + 1;
   if (g.twoD && tile.rho2d)
-    return ((n1 + r2_origin(n1, 64, 4) + 63) / 64) * ((n2 + r2_origin(n2, 32, 1) + 31) / 32);
+    return ((n1 + r2_origin(n1, 32, 4) + 31) / 32) * ((n2 + r2_origin(n2, 32, 1) + 31) / 32);
   if (g.twoD && tile.fuse2) {
     int o1, o2, nz, nx;
     return tf_origin(n1, n2, &o1, &o2, &nz, &nx) ? nz * nx : 0;

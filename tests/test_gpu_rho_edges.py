@@ -1,6 +1,6 @@
 """The 2D density step's tiles with the absorbing edges: remainders of the
-compute domain (ntaper 10: physical size + 20) modulo the 64 x 32 tile around
-the 10 cells that a line needs, one to three tiles across, against the oracle
+compute domain (ntaper 10: physical size + 20) modulo the tile around the 6
+cells that a line needs, one to seven tiles across, against the oracle
 bit for bit, traces and the whole padded field."""
 import numpy as np
 import pytest
