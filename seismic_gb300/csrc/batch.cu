@@ -452,17 +452,23 @@ __global__ void k_brho_grad(BatchTables t, int s_off) {
 
 // ---------------------------------------------------------------------------
 // The 2D variable-density step in one pass (FDderivatives.f90:601-657 and
-// the time update): each block owns a tile of 64 (z) x 32 (x) outputs.  At
+// the time update): each block owns a tile of 32 (z) x 32 (x) outputs.  At
 // its start it issues asynchronous 16-byte copies (cp.async, zero-filled
 // outside the padded array) into shared memory of what the gradients read:
-// u2 with an 8-cell halo (80 x 48) and delp with a 4-cell halo (72 x 40).
+// u2 with an 8-cell halo (48 x 48) and delp with a 4-cell halo (40 x 40).
 // It then forms the staggered gradients the tile's divergence reads - sz on
-// rows z0-4..z0+67 of the tile's columns, sx on columns x0-4..x0+35 of its
+// rows z0-4..z0+35 of the tile's columns, sx on columns x0-4..x0+35 of its
 // rows - with the operations and padding-cell rules of k_brho_grad, and
 // finally the divergence times v^2*rho and the rest of the point update
 // (step_tail), whose v, rho, u1, u0 and u_1 it reads straight into
 // registers.  Tiles at the boundary come first in the grid and, with `edges`,
 // end with the Higdon lines of their columns and rows.
+// Bound by the latency of the loads and of shared memory (the fields of
+// 771 x 2361 points fit in the L2), so by warps in flight and by the last
+// wave: 64 x 32 tiles with everything staged, two blocks per SM: 24.7 us per
+// step (and 8.2 for the edges); three blocks, the update's inputs from
+// registers: 22.0, the SMs busy for 69 % of it (2.1 waves); 32 x 32 tiles,
+// four blocks: 21 with the edges.
 // sz and sx never go through HBM: 32 bytes per point (u2, delp, v, rho, u1,
 // u0, u_1 read, u3 written) instead of the two passes' 52.
 // ---------------------------------------------------------------------------
@@ -475,7 +481,7 @@ constexpr int R2_SDP = R2_SU + R2_UX * R2_UZ;           // delp, R2_GX x R2_GZ
 constexpr int R2_SSZ = R2_SDP + R2_GX * R2_GZ;          // sz, R2_X x R2_GZ
 constexpr int R2_SSX = R2_SSZ + R2_X * R2_GZ;           // sx, R2_GX x R2_Z
 constexpr int R2_FLOATS = R2_SSX + R2_GX * R2_Z;
-constexpr size_t R2_SMEM = sizeof(float) * R2_FLOATS;   // 46 336 bytes
+constexpr size_t R2_SMEM = sizeof(float) * R2_FLOATS;   // 25 856 bytes
 // 16-byte chunks of the staged arrays.
 constexpr int R2_QU = R2_UX * (R2_UZ / 4), R2_QD = R2_GX * (R2_GZ / 4);
 constexpr int R2_PER_SM = 4;   // resident blocks
@@ -555,7 +561,7 @@ __global__ void __launch_bounds__(256, R2_PER_SM) k_brho2d(BatchTables t, int s_
   // checked when the batch is set up).
   auto off = [&](int i, int j) { return (i - lo1) + ld * (j - lo2); };
   // Every chunk starts a multiple of 4 rows from the padded array's first row
-  // (z0 - lo1 = 64 t + 4 - o1), so a chunk lies wholly inside a column's ld1 rows or wholly
+  // (z0 - lo1 = 32 t + 4 - o1), so a chunk lies wholly inside a column's ld1 rows or wholly
   // outside them; the arrays are 256-byte aligned and ld1 is a multiple of
   // 32, so every source address is 16-byte aligned.  Cells beyond the
   // padded array (zero-filled, or rows n1p..ld1-1 of a column) feed no value
@@ -597,7 +603,7 @@ __global__ void __launch_bounds__(256, R2_PER_SM) k_brho2d(BatchTables t, int s_
   // beyond (the fourth padding cell, which the reference reads and never
   // writes) and off the compute columns.  delp at (i, j) is
   // sdp[(j - x0 + 4) * R2_GZ + i - z0 + 4]; a face row or column that a
-  // padding cell of the tile needs lies inside the staged 72 x 40 block
+  // padding cell of the tile needs lies inside the staged 40 x 40 block
   // (a tile within 3 rows or columns of a face, or across it, stages it).
   // A tile whose gradient cells all lie inside the compute domain (most of
   // them) takes the 8th-order difference everywhere, without the per-cell

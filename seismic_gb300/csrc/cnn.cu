@@ -1094,6 +1094,9 @@ int cnn_forward(sw_cnn *n, int nz, int nx, int ny, const float *in, float *out) 
                                                                         n->a[0]);
   n->ctx->stats.launches_total++;
   if ((st = forward(n, nz, nx, ny))) return st;
+  TouchWhileBusy touch(n->ctx);
+  touch.add(out, npix * 4);
+  populate_touch(n->ctx);
   if ((e = cudaMemcpyAsync(out, n->out32, npix * 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
     return cnn_fail(n, e, "cnn output");
   return check_err(n);

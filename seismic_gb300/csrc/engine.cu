@@ -5,6 +5,9 @@
 // restates the reference in float, compiled with -ffp-contract=off, so the
 // weights are bit-identical to the reference formulas evaluated in IEEE
 // single precision.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
@@ -484,6 +487,18 @@ int upload(sw_ctx *c, const char *slot, const void *h, size_t bytes, void **d) {
   return SW_OK;
 }
 
+void populate_touch(sw_ctx *c) {
+  constexpr int kPopulateWrite = 23;   // MADV_POPULATE_WRITE (Linux 5.14)
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+  for (auto &t : c->touch) {
+    const uintptr_t a = ((uintptr_t)t.first + page - 1) / page * page;
+    const uintptr_t b = ((uintptr_t)t.first + t.second) / page * page;
+    // A kernel without it, or a mapping that it does not take, is left alone.
+    if (b > a) (void)madvise((void *)a, b - a, kPopulateWrite);
+  }
+  c->touch.clear();
+}
+
 int download(sw_ctx *c, void *h, const void *d, size_t bytes) {
   cudaError_t e = cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "download");
@@ -579,6 +594,9 @@ int sw_propagate(sw_ctx *c, const sw_prop_desc *d, const sw_prop_io *io) {
     dio.ref_dev = (float *)p;
   }
   dio.final_u2_host = io->final_u2;
+  TouchWhileBusy touch(c);
+  const Geom G = make_geom(d->g);
+  touch.add(io->final_u2, (size_t)G.n1p * G.n2p * G.n3p * sizeof(float));
   if ((st = propagate_dev(c, *d, dio))) return st;
   if (dio.nrec > 0 && (st = download(c, io->rec_trace, dio.rec_trace_dev, (size_t)dio.nrec * nt * sizeof(float))))
     return st;
@@ -636,6 +654,10 @@ static int two_pass(sw_ctx *c, const sw_genpar &g, const float *vel, const float
   if (st) return st;
   const int nt = g.nt, ntsnap = nt / g.snapi;
   const size_t nphys = (size_t)g.nz * g.nx * g.ny;
+  TouchWhileBusy touch(c);
+  touch.add(data_out, (size_t)std::max(nrec, 0) * nt * sizeof(float));
+  touch.add(image, nphys * sizeof(float));
+  touch.add(illum, nphys * sizeof(float));
   DevIO f;
   if ((st = upload_velocity(c, g, vel, "vel", &f.vel_pad))) return st;
   f.vel_phys_host = vel;

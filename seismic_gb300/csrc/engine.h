@@ -3,6 +3,7 @@
 
 #include <map>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <cudaTypedefs.h>
@@ -38,11 +39,33 @@ struct sw_ctx {
   sw_stats stats{};
   RunOpts run_opts;
   unsigned oc_epoch = 0;   // last packet epoch of the on-chip kernel's inbox
+  std::vector<std::pair<void *, size_t>> touch;   // see TouchWhileBusy
 };
 
 namespace swave {
 
 using ::RunOpts;
+
+// Has the pages of a call's host outputs mapped while the device works
+// (populate_touch, called once all launches of a phase are queued).  A copy
+// back into pages that the program has not touched faults them one by one
+// from the device: 27 ms for the 32 MB image and illumination of a
+// 100 x 200 x 200 migration, against 48 ms for all of its kernels.  The
+// contents stay as they are.  The list lives as long as the object.
+class TouchWhileBusy {
+ public:
+  explicit TouchWhileBusy(sw_ctx *c) : c_(c) {}
+  ~TouchWhileBusy() { c_->touch.clear(); }
+  TouchWhileBusy(const TouchWhileBusy &) = delete;
+  TouchWhileBusy &operator=(const TouchWhileBusy &) = delete;
+  void add(void *p, size_t bytes) {
+    if (p && bytes >= (1u << 18)) c_->touch.emplace_back(p, bytes);
+  }
+
+ private:
+  sw_ctx *c_;
+};
+void populate_touch(sw_ctx *c);
 
 struct InjPlan {
   int on = 0;

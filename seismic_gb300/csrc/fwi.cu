@@ -526,6 +526,11 @@ int sw_fwi_fct_gdt(sw_ctx *c, const sw_fwi_desc *dp, const float *vel, const flo
   cudaError_t e;
   const long long nfull = (long long)G.nz * G.nx * G.ny;
   const int nt = G.nt;
+  TouchWhileBusy touch(c);
+  touch.add(grad, nfull * sizeof(float));
+  touch.add(illum, nfull * sizeof(float));
+  for (int i = 0; i < nshot; ++i)
+    touch.add(shots[i].resid, (size_t)std::max(shots[i].nrec, 0) * nt * sizeof(float));
   void *p = nullptr;
   if ((st = upload(c, "fwi_vel", vel, nfull * sizeof(float), &p))) return st;
   const float *dvel = (const float *)p;

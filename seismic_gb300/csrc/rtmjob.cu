@@ -597,6 +597,8 @@ int sw_rtm_job_model(sw_rtm_job *j, int first, int count, float *const *data) {
     for (size_t q = 0; q < batch.size(); ++q)
       fwd[q] = forward_phase(j, j->shots[batch[q]], bufs[q], vhost[q], true);
     const uint64_t p0 = c->stats.points_updated;
+    TouchWhileBusy touch(c);
+    for (int k : batch) touch.add(data[k - first], (size_t)j->shots[k].s.nrec * j->shots[k].s.nt * 4);
     if ((st = run_phases(c, fwd, c->run_opts))) return st;
     j->points += c->stats.points_updated - p0;
     for (size_t q = 0; q < batch.size(); ++q) {
@@ -618,6 +620,9 @@ int sw_rtm_job_result(sw_rtm_job *j, float *image, float *illum, float *image_no
   cudaStream_t s = c->stream;
   const long long n = (long long)j->g.nz * j->g.nx * j->g.ny;
   int st = SW_OK;
+  TouchWhileBusy touch(c);
+  for (float *p : {image, illum, image_norm}) touch.add(p, n * 4);
+  populate_touch(c);
   if (image) SW_CK(cudaMemcpyAsync(image, j->image, n * 4, cudaMemcpyDeviceToHost, s));
   if (illum) SW_CK(cudaMemcpyAsync(illum, j->illum, n * 4, cudaMemcpyDeviceToHost, s));
   if (image_norm) {

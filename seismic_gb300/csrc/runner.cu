@@ -825,6 +825,7 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
       }
     }
   }
+  if (!c->touch.empty()) populate_touch(c);
   // Point updates actually performed (inactive shots skip their tiles).
   uint64_t upd = 0;
   for (auto &S : hs) upd += (uint64_t)S.npts * (uint64_t)S.nsteps;
