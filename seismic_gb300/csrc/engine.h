@@ -131,8 +131,8 @@ struct OcGroup {
   bool adj = false;
   int tile0 = 0, ncta = 0, cap = 0;
   int steps = 0, chunk = 0;   // steps of the longest member, steps per launch
-  size_t smem = 0, smem_v = 0;   // shared memory of a CTA, and with the velocity in it
-  bool vsm = false;
+  size_t smem = 0;              // shared memory of a CTA
+  bool vsm = false, pad = false;   // velocity in it; strides as OcArgs::pad
 };
 struct OcShotPlan {
   int cell0 = 0, ncell = 0;

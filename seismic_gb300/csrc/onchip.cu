@@ -79,7 +79,7 @@ bool shape_for(const Geom &g, int ncta, bool adj, int tcol, int tgrp, Shape *out
         t.TZ = a == 1 ? s.TZ : 4 * (a == 0 ? s.z[1] : NG - s.z[ntz - 1]);
         t.TX = e == 1 ? s.TX : 2 * (e == 0 ? s.x[1] : NP - s.x[ntx - 1]);
         t.nline = t.TX * (ntz == 1 ? 2 : a != 1) + t.TZ * (ntx == 1 ? 2 : e != 1);
-        fits = oc_smem_bytes(t, adj, false) <= kSmemLimit;
+        fits = oc_smem_bytes(t, adj, false, false) <= kSmemLimit;
       }
     if (!fits) continue;
     const long long cost = (long long)s.TZ * s.TX + 8LL * (s.TZ + s.TX);
@@ -203,6 +203,7 @@ bool oc_plan(sw_ctx *c, const std::vector<PhaseShot> &shots, const std::vector<G
     g.members = m;
     g.adj = adj[m[0]] != 0;
     g.tile0 = (int)R.tiles.size();
+    size_t smem[4] = {0, 0, 0, 0};   // [vsm + 2 pad]
     std::vector<int> n(m.size());
     int used = 0;
     for (size_t q = 0; q < m.size(); ++q) used += n[q] = cmin[m[q]];
@@ -304,11 +305,11 @@ bool oc_plan(sw_ctx *c, const std::vector<PhaseShot> &shots, const std::vector<G
                     cb = std::min(t.c0 + t.TX, inj[b].bj0 - gg.lo2 + P.ncol);
           if (P.nent && ra < rb && ca < cb) {
             t.nterm = P.M * (cb - ca) * (rb - ra);
-            if (oc_smem_bytes(t, g.adj, false) > kSmemLimit) t.nterm = 0;
+            if (oc_smem_bytes(t, g.adj, false, false) > kSmemLimit) t.nterm = 0;
           }
-          if (oc_smem_bytes(t, g.adj, false) > kSmemLimit) return false;
-          g.smem = std::max(g.smem, oc_smem_bytes(t, g.adj, false));
-          g.smem_v = std::max(g.smem_v, oc_smem_bytes(t, g.adj, true));
+          if (oc_smem_bytes(t, g.adj, false, false) > kSmemLimit) return false;
+          for (int k = 0; k < 4; ++k)
+            smem[k] = std::max(smem[k], oc_smem_bytes(t, g.adj, k & 1, k & 2));
           R.tiles.push_back(t);
         }
       P.ncell = (int)R.cells.size() - P.cell0;
@@ -334,8 +335,13 @@ bool oc_plan(sw_ctx *c, const std::vector<PhaseShot> &shots, const std::vector<G
       g.steps = std::max(g.steps, nsteps[b]);
     }
     g.ncta = (int)R.tiles.size() - g.tile0;
-    g.vsm = g.smem_v <= kSmemLimit;
-    if (g.vsm) g.smem = g.smem_v;
+    // The velocity on the chip before strides without bank conflicts.
+    for (int k : {0, 2, 1, 3})
+      if (smem[k] <= kSmemLimit) {
+        g.smem = smem[k];
+        g.vsm = k & 1;
+        g.pad = k & 2;
+      }
     size_t freeb = 0, totalb = 0;
     if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) return false;
     size_t held = 0;
@@ -440,6 +446,7 @@ int oc_run(sw_ctx *c, const std::vector<ShotDev> &hs, const ShotDev *dshots, OcR
       a.cap = g.cap;
       a.rigid = rigid ? 1 : 0;
       a.vsm = g.vsm ? 1 : 0;
+      a.pad = g.pad ? 1 : 0;
       a.err = derr;
       for (int s0 = 0; s0 < g.steps; s0 += g.chunk) {
         a.s0 = s0;

@@ -71,6 +71,7 @@ struct OcArgs {
   int s0, s1;            // steps of the launch (a shot stops at its own last step)
   unsigned epoch0;       // packets of step s carry epoch0 + (s - s0) + 1
   int rigid, vsm;        // vsm: the tiles' velocity is kept in shared memory
+  int pad;               // see oc_strides
   int *err;
 };
 
@@ -80,15 +81,26 @@ __host__ __device__ inline int oc_stride(int rows) {
   const int q = (rows + 3) / 4;
   return 4 * (q | 1);
 }
+// Strides of the arrays with (hs) and without (cs) the border.  With pad
+// they are the same modulo 4 units: the order of the work items that keeps
+// the accesses of 8 lanes in different banks in one array then does so in
+// the others.  Without room for it (2 or 4 units per column of some arrays)
+// the bordered arrays alone are free of conflicts.
+__host__ __device__ inline void oc_strides(int TZ, bool adj, bool pad, int *hs, int *cs) {
+  *hs = oc_stride(TZ + 8);
+  *cs = oc_stride(TZ);
+  if (pad && adj) *hs = *cs + 16;
+  if (pad && !adj) *cs = *hs;
+}
 // Dynamic shared memory of a tile: its levels (and velocity, vsm) and work items, and with them
 // its injection terms (two parities) and edge lines (coefficients, velocity).
-__host__ __device__ inline size_t oc_smem_bytes(int TZ, int TX, bool adj, bool vsm) {
-  const size_t h = (size_t)oc_stride(TZ + 8) * (TX + 8), c = (size_t)oc_stride(TZ) * TX;
-  const size_t items = (size_t)(TZ / 4) * (TX / 2);
-  return 4 * ((adj ? 4 * c + 2 * h : 4 * h) + (vsm ? c : 0) + items) + 16;
-}
-__host__ __device__ inline size_t oc_smem_bytes(const OcTile &t, bool adj, bool vsm) {
-  return oc_smem_bytes(t.TZ, t.TX, adj, vsm) + 8 * (size_t)t.nterm + (adj ? 64 : 32) * (size_t)t.nline;
+__host__ __device__ inline size_t oc_smem_bytes(const OcTile &t, bool adj, bool vsm, bool pad) {
+  int hs, cs;
+  oc_strides(t.TZ, adj, pad, &hs, &cs);
+  const size_t h = (size_t)hs * (t.TX + 8), c = (size_t)cs * t.TX;
+  const size_t items = (size_t)(t.TZ / 4) * (t.TX / 2);
+  return 4 * ((adj ? 4 * c + 2 * h : 4 * h) + (vsm ? c : 0) + items) + 16 +
+         8 * (size_t)t.nterm + (adj ? 64 : 32) * (size_t)t.nline;
 }
 
 __device__ __forceinline__ void oc_put(ulonglong2 *p, float a, float b, unsigned epoch) {
@@ -157,7 +169,7 @@ __device__ __forceinline__ float *oc_save_slot(const ShotDev &S, const OcShot &O
 template <bool ADJ>
 __global__ void __launch_bounds__(OC_THREADS, OC_PER_SM) k_onchip2d(OcArgs A) {
   extern __shared__ __align__(16) float oc_sm[];
-  __shared__ int n_items[2];
+  __shared__ int n_items[2], n_class[16], n_rank[16];
   __shared__ volatile int abort_flag;
   __shared__ ShotDev S;
   const OcTile T = A.tiles[blockIdx.x];
@@ -171,7 +183,8 @@ __global__ void __launch_bounds__(OC_THREADS, OC_PER_SM) k_onchip2d(OcArgs A) {
   __syncthreads();
   const int n1p = S.g.n1p, n2p = S.g.n2p, ld1 = S.g.ld1;
   const int TZ = T.TZ, TX = T.TX, r0 = T.r0, c0 = T.c0;
-  const int HS = oc_stride(TZ + 8), CS = oc_stride(TZ);
+  int HS, CS;
+  oc_strides(TZ, ADJ, A.pad != 0, &HS, &CS);
   const int hsz = HS * (TX + 8);
   // Levels: forward tiles keep them with the border (the stencil reads u2),
   // adjoint tiles without it (the stencil reads w).
@@ -222,9 +235,16 @@ __global__ void __launch_bounds__(OC_THREADS, OC_PER_SM) k_onchip2d(OcArgs A) {
   // lines alone; of the x zones only the rows the z lines start from (two
   // beyond each z zone) are computed, in the first list.
   const int zlo = hig ? 8 : 4, zhi = hig ? n1p - 9 : n1p - 5;
+  // Within a list they go round the 8 classes of (row group + column offset
+  // in 16-byte units) modulo 8, so that a quarter warp's 16-byte accesses
+  // meet 32 different banks whatever the stride and the holes of the lists.
+  // In order of rows the items of a quarter warp took 2.6 passes of the
+  // shared-memory pipe per access on average, which bound the step.
   if (warp == 0) {
-    int n = 0;
-    for (int list = 0; list < 2; ++list) {
+    if (lane < 16) n_class[lane] = n_rank[lane] = 0;
+    __syncwarp();
+    int n0 = 0;
+    for (int pass = 0; pass < 2; ++pass) {
       for (int q0 = 0; q0 < NG * NP; q0 += 32) {
         const int q = q0 + lane, p = q / NG, g = q % NG;
         const int R = r0 + 4 * g, C = c0 + NC * p;
@@ -241,12 +261,35 @@ __global__ void __launch_bounds__(OC_THREADS, OC_PER_SM) k_onchip2d(OcArgs A) {
                            (NC * p < 4 && T.nb[0] >= 0) ||
                            (NC * p >= TX - 4 && T.nb[1] >= 0) ||
                            (hig && ((C <= 9 && C + NC > 8) || (C <= n2p - 9 && C + NC > n2p - 10)));
-        use = use && first == (list == 0);
-        const unsigned m = __ballot_sync(0xffffffffu, use);
-        if (use) items[n + __popc(m & ((1u << lane) - 1))] = g | (p << 8) | (f << 16);
-        n += __popc(m);
+        const int cls = (g + p * (NC * HS / 4)) & 7;
+        const int key = use ? cls + (first ? 0 : 8) : -1;
+        const unsigned m = __match_any_sync(0xffffffffu, key);
+        const int before = __popc(m & ((1u << lane) - 1));
+        int *const count = pass ? n_rank : n_class;
+        if (pass && use) {
+          // The items of the list that come earlier in the round.
+          const int rank = n_rank[key] + before;
+          int pos = first ? 0 : n0;
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            pos += min(n_class[(key & 8) + k], rank + (k < cls ? 1 : 0));
+          items[pos] = g | (p << 8) | (f << 16);
+        }
+        __syncwarp();
+        if (use && before == 0) count[key] += __popc(m);
+        __syncwarp();
       }
-      if (lane == 0) n_items[list] = n;
+      if (pass == 0) {
+        int n = 0;
+        for (int k = 0; k < 16; ++k) {
+          n += n_class[k];
+          if (k == 7) n0 = n;
+        }
+        if (lane == 0) {
+          n_items[0] = n0;
+          n_items[1] = n;
+        }
+      }
     }
     if (lane == 0) abort_flag = 0;
   }
