@@ -81,6 +81,15 @@ __device__ __forceinline__ void cnn_tma4(void *dst, const CUtensorMap *map, int 
       "r"(umma_su32(bar))
       : "memory");
 }
+// The kernels of a pass follow one another by programmatic launches: a
+// kernel's CTAs start as those of the one before leave, set themselves up
+// and wait here before they touch a tensor.  Tensor memory is allocated
+// before the successor is let go, so a CTA that holds some and waits never
+// stands in the way of one that it waits for.
+__device__ __forceinline__ void cnn_chain() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 // Instruction descriptor with both operands MN-major (transposed).
 __host__ __device__ constexpr uint32_t umma_idesc_bf16_mn(int M, int N) {
   return umma_idesc_bf16(M, N) | (1u << 15) | (1u << 16);
@@ -214,6 +223,7 @@ __global__ void __launch_bounds__(kWsThreads, 2)
   umma_fence_before();
   __syncthreads();
   umma_fence_after();
+  cnn_chain();
   const unsigned tmem = tmem_base;
   const int first = blockIdx.x, stride = gridDim.x;
   const int nmine = first < A.ntiles ? (A.ntiles - 1 - first) / stride + 1 : 0;
@@ -443,6 +453,7 @@ __global__ void __launch_bounds__(kWsThreads, 1)
   umma_fence_before();
   __syncthreads();
   umma_fence_after();
+  cnn_chain();
   const unsigned tmem = tmem_base;
   const int first = blockIdx.x, stride = gridDim.x;
   const int nmine = first < A.ntiles ? (A.ntiles - 1 - first) / stride + 1 : 0;
@@ -590,6 +601,7 @@ __global__ void __launch_bounds__(kSumW * kMaxC) k_wgrad_sum(const SumArgs A) {
   const int tap = blockIdx.x, co = blockIdx.y, l = blockIdx.z;
   const int ci = threadIdx.x % kMaxC, w = threadIdx.x / kMaxC;
   const int Cin = A.Cin[l], Cout = A.Cout[l], taps = A.taps;
+  cnn_chain();
   if (co >= Cout) return;
   const bool use = tap == taps ? ci == 0 : ci < Cin;
   const float *P = A.part[l] + (size_t)tap * kMaxC * kMaxC + co * kMaxC + ci;
@@ -610,6 +622,7 @@ __global__ void __launch_bounds__(kSumW * kMaxC) k_wgrad_sum(const SumArgs A) {
 __global__ void k_pack_input(const float *__restrict__ in, int C, int npix,
                              __nv_bfloat16 *__restrict__ out) {
   const int g = blockIdx.y;
+  cnn_chain();
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
     float v[8];
 #pragma unroll
@@ -623,11 +636,13 @@ __global__ void k_pack_input(const float *__restrict__ in, int C, int npix,
 // Mean-square loss of a one-channel output: the output gradient
 // (out - target) / npix as BF16 in channel 0 of a 16-channel tensor (two
 // planes, zero elsewhere), and per-block FP64 partial sums of
-// (out - target)^2.
+// (out - target)^2.  Few blocks: their FP64 tree sums cost more than the
+// pixels (1024 blocks: 9.3 us for 301 x 901).
 __global__ void k_loss(const float *__restrict__ out, const float *__restrict__ tgt, int npix,
                        __nv_bfloat16 *__restrict__ db, double *__restrict__ part) {
   __shared__ double red[8];
   double s = 0.0;
+  cnn_chain();
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
     const float e = out[p] - tgt[p];
     s += (double)e * (double)e;
@@ -713,14 +728,30 @@ int num_sms(int dev) {
   return n;
 }
 
+// A kernel of the chain (cnn_chain).
+template <typename... P, typename... Q>
+cudaError_t launch_chained(void (*k)(P...), dim3 grid, int block, size_t smem, cudaStream_t s,
+                           const Q &...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
 template <class K>
 cudaError_t launch_big(K kernel, int grid, size_t smem, cudaStream_t s, const CUtensorMap &m0,
                        const ConvArgs &a) {
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return e;
-  kernel<<<grid, kWsThreads, smem, s>>>(m0, a);
-  return cudaGetLastError();
+  return launch_chained(kernel, dim3(grid), kWsThreads, smem, s, m0, a);
 }
 
 // One convolution: input tensor (Cs channels) -> MODE's outputs.
@@ -787,14 +818,13 @@ cudaError_t launch_wgrad(int dev, const __nv_bfloat16 *a, int Cin, const __nv_bf
     e = cudaFuncSetAttribute(k_wgrad_umma<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
     if (e != cudaSuccess) return e;
-    k_wgrad_umma<16><<<grid, kWsThreads, smem, s>>>(ma, md, w);
+    return launch_chained(k_wgrad_umma<16>, dim3(grid), kWsThreads, smem, s, ma, md, w);
   } else {
     e = cudaFuncSetAttribute(k_wgrad_umma<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
     if (e != cudaSuccess) return e;
-    k_wgrad_umma<32><<<grid, kWsThreads, smem, s>>>(ma, md, w);
+    return launch_chained(k_wgrad_umma<32>, dim3(grid), kWsThreads, smem, s, ma, md, w);
   }
-  return cudaGetLastError();
 }
 
 }  // namespace
@@ -962,7 +992,7 @@ int gradient(sw_cnn *n, int nbatch, int nz, int nx, int ny, const float *in, con
   if (st) return st;
   cudaError_t e;
   if ((e = cudaMemsetAsync(n->g, 0, n->nw * 4, s)) != cudaSuccess) return cnn_fail(n, e, "cnn");
-  const int lblocks = (int)std::min<size_t>(1024, (npix + 255) / 256);
+  const int lblocks = (int)std::min<size_t>(304, (npix + 255) / 256);
   double lsum = 0.0;
   std::vector<double> hp(lblocks);
   for (int ib = 0; ib < nbatch; ++ib) {
@@ -978,7 +1008,9 @@ int gradient(sw_cnn *n, int nbatch, int nz, int nx, int ny, const float *in, con
     if ((st = forward(n, nz, nx, ny))) return st;
     // d loss / d output (one channel), FP64 loss partials.
     int cur = 0;
-    k_loss<<<lblocks, 256, 0, s>>>(n->out32, n->tgt, (int)npix, n->dz[cur], n->lpart);
+    if ((e = launch_chained(k_loss, dim3(lblocks), 256, 0, s, n->out32, n->tgt, (int)npix,
+                            n->dz[cur], n->lpart)) != cudaSuccess)
+      return cnn_fail(n, e, "cnn loss");
     n->ctx->stats.launches_total++;
     SumArgs sum;
     sum.taps = T;
@@ -1014,9 +1046,10 @@ int gradient(sw_cnn *n, int nbatch, int nz, int nx, int ny, const float *in, con
         return cnn_fail(n, e, "cnn dgrad");
       cur ^= 1;
     }
-    k_wgrad_sum<<<dim3(T + 1, kMaxC, n->nl), kSumW * kMaxC, 0, s>>>(sum);
+    if ((e = launch_chained(k_wgrad_sum, dim3(T + 1, kMaxC, n->nl), kSumW * kMaxC, 0, s, sum)) !=
+        cudaSuccess)
+      return cnn_fail(n, e, "cnn backward");
     n->ctx->stats.launches_total++;
-    if ((e = cudaGetLastError()) != cudaSuccess) return cnn_fail(n, e, "cnn backward");
     if ((e = cudaMemcpyAsync(hp.data(), n->lpart, lblocks * sizeof(double),
                              cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
