@@ -136,6 +136,71 @@ __global__ void k_triangle(int n12, int nr, int nlines, int lines_inner, long lo
   for (int i = 0; i < n12; ++i) vv[base + i * estride] = tt[i];
 }
 
+// The same in shared memory, in place: a block takes `nl` lines.  All threads
+// do what is element by element (the differences, the divisions, the ends);
+// one thread per line runs the two chains of additions, whose order gives
+// the sums their bits.  One thread per line with its vectors in global
+// memory, as above, took 1.7 ms per axis for 301 x 901 points.
+constexpr int kTriLines = 8, kTriThreads = 256;
+constexpr size_t kTriSmem = 200 * 1024;
+__host__ __device__ inline size_t tri_stride(int n12, int nr) {
+  return (size_t)(n12 + 2 * nr) | 1;   // lines start in different banks
+}
+__global__ void __launch_bounds__(kTriThreads) k_triangle_sm(int n12, int nr, int nlines, int nl,
+                                                             int lines_inner,
+                                                             long long lstride_in,
+                                                             long long lstride_out,
+                                                             long long estride, float *u) {
+  extern __shared__ float tri_sm[];
+  const int S = (int)tri_stride(n12, nr), tid = threadIdx.x;
+  float *X = tri_sm, *B = tri_sm + (size_t)nl * S;
+  const int l0 = blockIdx.x * nl, mine = min(nl, nlines - l0);
+  if (n12 == 1) return;   // the line as it is
+  auto base = [&](int k) {
+    const int l = l0 + k;
+    return (long long)(l % lines_inner) * lstride_in + (long long)(l / lines_inner) * lstride_out;
+  };
+  // Neighbouring threads on neighbouring addresses along either axis.
+  const bool by_line = estride != 1;
+  auto each = [&](int n, auto f) {
+    for (int q = tid; q < n * mine; q += kTriThreads) {
+      if (by_line) f(q % mine, q / mine);
+      else f(q / n, q % n);
+    }
+  };
+  each(n12, [&](int k, int i) { X[k * S + i] = u[base(k) + i * estride]; });
+  int nx = n12;
+  for (int pass = 0; pass < 2; ++pass) {
+    __syncthreads();
+    if (tid < mine) {
+      const float *x = X + tid * S;
+      float *b = B + tid * S, v = x[0];
+      b[0] = v;
+#pragma unroll 8
+      for (int i = 1; i < nx; ++i) {
+        v = v + x[i];
+        b[i] = v;
+      }
+    }
+    __syncthreads();
+    each(nx + nr - 1, [&](int k, int i) {
+      const float *b = B + k * S;
+      float y = b[min(i, nx - 1)];
+      if (i >= nr) y = y - b[min(i - nr, nx - 1)];
+      X[k * S + i] = y / (float)nr;
+    });
+    nx += nr - 1;
+  }
+  __syncthreads();
+  each(n12, [&](int k, int i) {
+    const float *q = X + k * S;
+    float t = q[i + nr - 1];
+    if (i <= nr - 2) t = t + q[nr - 2 - i];
+    if (n12 - i <= nr - 1) t = t + q[2 * n12 + nr - 2 - i];
+    u[base(k) + i * estride] = t;
+  });
+}
+
 // ---------------------------------------------------------------------------
 // FP64 vector kernels for the L-BFGS
 // ---------------------------------------------------------------------------
@@ -769,14 +834,26 @@ int sw_fwi_fct_gdt(sw_ctx *c, const sw_fwi_desc *dp, const float *vel, const flo
   c->stats.launches_total += 3;
   // triangle2 (Smoothing.f90:87-138); y pass with rect3/n3 (see the oracle).
   const int n1 = G.nz, n2 = G.nx, n3 = G.ny;
-  float *tmpb = (float *)dbuf(c, "tri_out", nfull * sizeof(float), &st);
-  if (!tmpb) return st;
   auto tri = [&](int n12, int nr, int nlines, int inner, long long ls_in, long long ls_out,
                  long long es) -> int {
     if (nr < 1 || nr > n12) return fail(c, SW_BAD_PARAM, "triangle radius %d out of range", nr);
+    const size_t line = 2 * sizeof(float) * tri_stride(n12, nr);
+    if (line <= kTriSmem) {   // lines of up to 25000 points, 3200 in eights
+      const int nl = (int)std::min<size_t>(kTriLines, kTriSmem / line);
+      cudaError_t ee = cudaFuncSetAttribute(
+          k_triangle_sm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTriSmem);
+      if (ee == cudaSuccess) {
+        k_triangle_sm<<<(nlines + nl - 1) / nl, kTriThreads, nl * line, s>>>(
+            n12, nr, nlines, nl, inner, ls_in, ls_out, es, dgrad);
+        ee = cudaGetLastError();
+      }
+      c->stats.launches_total++;
+      return ee == cudaSuccess ? SW_OK : cuda_fail(c, ee, "triangle");
+    }
     const size_t per = 4ull * (size_t)(n12 + 2 * nr);
     float *scr = (float *)dbuf(c, "tri_scr", per * (size_t)nlines * sizeof(float), &st);
-    if (!scr) return st;
+    float *tmpb = (float *)dbuf(c, "tri_out", nfull * sizeof(float), &st);
+    if (!scr || !tmpb) return st;
     k_triangle<<<(nlines + 127) / 128, 128, 0, s>>>(n12, nr, nlines, inner, ls_in, ls_out, es,
                                                     dgrad, tmpb, scr);
     cudaError_t ee = cudaMemcpyAsync(dgrad, tmpb, nfull * sizeof(float), cudaMemcpyDeviceToDevice, s);
