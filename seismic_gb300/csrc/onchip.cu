@@ -97,7 +97,7 @@ int num_sms(int dev) {
   return n;
 }
 
-template <bool ADJ>
+template <bool ADJ, bool VSM>
 cudaError_t launch(const OcArgs &a, int ncta, size_t smem, cudaStream_t s) {
   // The shared-memory opt-in is a per-device function attribute.
   static unsigned long long attr_set = 0;
@@ -105,7 +105,7 @@ cudaError_t launch(const OcArgs &a, int ncta, size_t smem, cudaStream_t s) {
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev >= 64 || !(attr_set & (1ull << dev))) {
-    e = cudaFuncSetAttribute(k_onchip2d<ADJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(k_onchip2d<ADJ, VSM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kSmemLimit);
     if (e != cudaSuccess) return e;
     if (dev < 64) attr_set |= 1ull << dev;
@@ -113,7 +113,7 @@ cudaError_t launch(const OcArgs &a, int ncta, size_t smem, cudaStream_t s) {
   // Cooperative: the CTAs wait for one another, so all must be resident.
   OcArgs arg = a;
   void *args[] = {&arg};
-  return cudaLaunchCooperativeKernel((const void *)k_onchip2d<ADJ>, dim3(ncta), dim3(OC_THREADS),
+  return cudaLaunchCooperativeKernel((const void *)k_onchip2d<ADJ, VSM>, dim3(ncta), dim3(OC_THREADS),
                                      args, smem, s);
 }
 
@@ -445,7 +445,6 @@ int oc_run(sw_ctx *c, const std::vector<ShotDev> &hs, const ShotDev *dshots, OcR
       a.inbox = (ulonglong2 *)R.d_inbox;
       a.cap = g.cap;
       a.rigid = rigid ? 1 : 0;
-      a.vsm = g.vsm ? 1 : 0;
       a.pad = g.pad ? 1 : 0;
       a.err = derr;
       for (int s0 = 0; s0 < g.steps; s0 += g.chunk) {
@@ -461,7 +460,10 @@ int oc_run(sw_ctx *c, const std::vector<ShotDev> &hs, const ShotDev *dshots, OcR
           ++*launches;
         }
         if (c->profiling) SW_CK(cudaEventRecord(ev[0], s));
-        e = g.adj ? launch<true>(a, g.ncta, g.smem, s) : launch<false>(a, g.ncta, g.smem, s);
+        e = g.adj ? (g.vsm ? launch<true, true>(a, g.ncta, g.smem, s)
+                           : launch<true, false>(a, g.ncta, g.smem, s))
+                  : (g.vsm ? launch<false, true>(a, g.ncta, g.smem, s)
+                           : launch<false, false>(a, g.ncta, g.smem, s));
         if (e != cudaSuccess) return cuda_fail(c, e, "on-chip propagation");
         ++*launches;
         if (c->profiling) {

@@ -70,7 +70,7 @@ struct OcArgs {
   int cap;
   int s0, s1;            // steps of the launch (a shot stops at its own last step)
   unsigned epoch0;       // packets of step s carry epoch0 + (s - s0) + 1
-  int rigid, vsm;        // vsm: the tiles' velocity is kept in shared memory
+  int rigid;
   int pad;               // see oc_strides
   int *err;
 };
@@ -166,7 +166,7 @@ __device__ __forceinline__ float *oc_save_slot(const ShotDev &S, const OcShot &O
   return nullptr;
 }
 
-template <bool ADJ>
+template <bool ADJ, bool VSM>
 __global__ void __launch_bounds__(OC_THREADS, OC_PER_SM) k_onchip2d(OcArgs A) {
   extern __shared__ __align__(16) float oc_sm[];
   __shared__ int n_items[2], n_class[16], n_rank[16];
@@ -191,8 +191,8 @@ __global__ void __launch_bounds__(OC_THREADS, OC_PER_SM) k_onchip2d(OcArgs A) {
   const int US = ADJ ? CS : HS, UO = ADJ ? 0 : 4 * HS + 4, usz = ADJ ? CS * TX : hsz;
   float *const lev0 = oc_sm;
   float *const w0 = oc_sm + 4 * usz;
-  float *const V = w0 + (ADJ ? 2 * hsz : 0);   // the velocity, if there is room
-  int *const items = reinterpret_cast<int *>(V + (A.vsm ? CS * TX : 0));
+  float *const V = w0 + (ADJ ? 2 * hsz : 0);   // its square, if there is room (VSM)
+  int *const items = reinterpret_cast<int *>(V + (VSM ? CS * TX : 0));
   const bool hig = !A.rigid;
   const int se = min(A.s1, S.nsteps);   // this shot's steps: [s0, se)
   if (A.s0 >= se) return;               // uniform over the shot's CTAs
@@ -209,10 +209,10 @@ __global__ void __launch_bounds__(OC_THREADS, OC_PER_SM) k_onchip2d(OcArgs A) {
       const long long off = (long long)R + (long long)ld1 * C;
       const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
       float4 v2 = zero;
-      if (in && (ADJ || (A.vsm && core))) {
+      if (in && (ADJ || (VSM && core))) {
         const float4 v = oc_ld4(S.vel + off);
-        if (A.vsm && core) *reinterpret_cast<float4 *>(V + c * CS + 4 * g) = v;
         v2 = make_float4(v.x * v.x, v.y * v.y, v.z * v.z, v.w * v.w);
+        if (VSM && core) *reinterpret_cast<float4 *>(V + c * CS + 4 * g) = v2;
       }
 #pragma unroll
       for (int l = 0; l < 4; ++l) {
@@ -430,11 +430,11 @@ __global__ void __launch_bounds__(OC_THREADS, OC_PER_SM) k_onchip2d(OcArgs A) {
       const int rl = 4 * (e & 255), cl = NC * ((e >> 8) & 255);
       const float *col0 = op + (cl + 4) * HS + rl + 4;
       const int nrow = zhi - (r0 + rl) + 1;   // rows to store
-      float4 vel[NC];
+      float4 vel[NC];   // the square of the velocity with VSM
 #pragma unroll
       for (int cc = 0; cc < NC; ++cc)
-        vel[cc] = A.vsm ? oc_ld4(V + (cl + cc) * CS + rl)
-                        : oc_ld4(vel0 + ld1 * min(cl + cc, n2p - 1 - c0) + rl);
+        vel[cc] = VSM ? oc_ld4(V + (cl + cc) * CS + rl)
+                      : oc_ld4(vel0 + ld1 * min(cl + cc, n2p - 1 - c0) + rl);
       // Columns cl-4 .. cl+NC+3, each loaded once.
       float4 N[NC + 8];
 #pragma unroll
@@ -445,16 +445,20 @@ __global__ void __launch_bounds__(OC_THREADS, OC_PER_SM) k_onchip2d(OcArgs A) {
         const float4 za = oc_ld4(col0 + cc * HS - 4), zc = oc_ld4(col0 + cc * HS + 4);
         const float4 zb = N[4 + cc];
         const P2 P[6] = {lo2(za), hi2(za), lo2(zb), hi2(zb), lo2(zc), hi2(zc)};
-        P2 Q[5];   // rows (2k + 1, 2k + 2)
-#pragma unroll
-        for (int k = 0; k < 5; ++k) Q[k] = p2(P[k].y, P[k + 1].x);
+        // Pairs of rows at odd distances straddle the loaded pairs: scalar
+        // sums there cost fewer instructions than the moves to form pairs.
+        const float zr[12] = {za.x, za.y, za.z, za.w, zb.x, zb.y,
+                              zb.z, zb.w, zc.x, zc.y, zc.z, zc.w};
         P2 tzz[2], txx[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
+          const int m = 4 + 2 * h;
           P2 a = s_mul(c0z, P[2 + h]);
-          a = p_add(a, s_mul(c1z, p_add(Q[2 + h], Q[1 + h])));
+          a = p_add(a, p2(__fmul_rn(c1z, zr[m + 1] + zr[m - 1]),
+                          __fmul_rn(c1z, zr[m + 2] + zr[m])));
           a = p_add(a, s_mul(c2z, p_add(P[3 + h], P[1 + h])));
-          a = p_add(a, s_mul(c3z, p_add(Q[3 + h], Q[h])));
+          a = p_add(a, p2(__fmul_rn(c3z, zr[m + 3] + zr[m - 3]),
+                          __fmul_rn(c3z, zr[m + 4] + zr[m - 2])));
           a = p_add(a, s_mul(c4z, p_add(P[4 + h], P[h])));
           tzz[h] = a;
           txx[h] = s_mul(cx[0], P[2 + h]);
@@ -465,8 +469,8 @@ __global__ void __launch_bounds__(OC_THREADS, OC_PER_SM) k_onchip2d(OcArgs A) {
           txx[0] = p_add(txx[0], s_mul(cx[l], p_add(lo2(rp), lo2(rm))));
           txx[1] = p_add(txx[1], s_mul(cx[l], p_add(hi2(rp), hi2(rm))));
         }
-        v2c[cc][0] = p_mul(lo2(vel[cc]), lo2(vel[cc]));
-        v2c[cc][1] = p_mul(hi2(vel[cc]), hi2(vel[cc]));
+        v2c[cc][0] = VSM ? lo2(vel[cc]) : p_mul(lo2(vel[cc]), lo2(vel[cc]));
+        v2c[cc][1] = VSM ? hi2(vel[cc]) : p_mul(hi2(vel[cc]), hi2(vel[cc]));
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           svc[cc][h] = p_add(txx[h], tzz[h]);
@@ -507,7 +511,8 @@ __global__ void __launch_bounds__(OC_THREADS, OC_PER_SM) k_onchip2d(OcArgs A) {
           if (cnt <= S.ntsnap && j >= 1 && j <= S.g.nx) {
             const float *ws = S.wave + (long long)(cnt - 1) * nphys;
             const float taper = S.taperx ? S.taperx[j - 1] * S.tapery[0] : 1.f;
-            const float vc[4] = {vel[cc].x, vel[cc].y, vel[cc].z, vel[cc].w};
+            const float4 vq = VSM ? oc_ld4(vel0 + ld1 * (cl + cc) + rl) : vel[cc];
+            const float vc[4] = {vq.x, vq.y, vq.z, vq.w};
             float r[4] = {sv[0].x, sv[0].y, sv[1].x, sv[1].y};
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
