@@ -341,9 +341,9 @@ def main():
     # Shots of this rank: rank r takes every ws-th shot of the survey.
     from seismic_gb300 import dist as sdist
     mine = [shots[i] for i in sdist.shard(len(shots), rank, ws)]
-    # Shots per step and launch shape: the autotuner (batch candidates
-    # capped by what HBM admits at full record length, timed on truncated
-    # records; then the launch shape at that batch), untimed.
+    # 16 shots per step.  Shots per batch and launch shape: the autotuner
+    # (batch candidates capped by what HBM admits at full record length, timed
+    # on truncated records; then the launch shape at that batch), untimed.
     tune = None
     if not args.no_tune:
         from seismic_gb300 import autotune
@@ -353,7 +353,8 @@ def main():
         if args.no_graph:
             ctx.set_tuning(use_graph=0)
         log(f"[rank {rank}] autotune: {tune}")
-    B = args.shots_per_step or (tune["batch"] if tune else 16)
+    B = args.shots_per_step or 16
+    nbatch = min(B, tune["batch"]) if tune else B
     nsteps = args.warmup + args.steps
     per_step = [mine[(k * B + q) % len(mine)] for k in range(nsteps) for q in range(B)]
     # Observed data: batched forward modelling on each shot's window (untimed).
@@ -366,7 +367,7 @@ def main():
             distinct[key] = None
             uniq.append(s)
     mj = sw.RTMJob(ctx, g, vel, w, [{"sou": s["sou"], "rec": s["rec"], "nt": s["nt"]} for s in uniq])
-    mj.set_batch(B)
+    mj.set_batch(nbatch)
     for s, d in zip(uniq, mj.model()):
         distinct[float(s["sou"][1])] = d
     mj.close()
@@ -374,7 +375,7 @@ def main():
     job_shots = [{"sou": s["sou"], "rec": s["rec"], "data": distinct[float(s["sou"][1])]}
                  for s in per_step]
     job = sw.RTMJob(ctx, g, vel, w, job_shots)
-    job.set_batch(B)
+    job.set_batch(nbatch)
 
     def barrier():
         if ws > 1:
@@ -433,9 +434,14 @@ def main():
     # algorithmic bytes over every fused-kernel launch of a smaller RTM batch
     # (profiles/step_kernel_traffic.json) times this run's algorithmic bytes.
     algo_per_launch = st["step_bytes"] / nl
+    # Shots that fit on the chip take many steps per launch (k_onchip2d); the
+    # figures are then per step, and the 24 B per update are what a kernel
+    # that reads its levels from HBM would move: the launch itself moves only
+    # snapshots, terms and borders.
+    onchip = st["launches_total"] < st["step_kernel_timed"]
     traffic = None
     prof_json = os.path.join(ROOT, "profiles", "step_kernel_traffic.json")
-    if os.path.exists(prof_json):
+    if os.path.exists(prof_json) and not onchip:
         try:
             traffic = float(json.load(open(prof_json))["dram_per_algorithmic"]) * algo_per_launch
         except Exception:
@@ -453,7 +459,7 @@ def main():
         torch.cuda.synchronize()
         t0 = time.perf_counter()
         j2 = sw.RTMJob(ctx, g, hvel, hw, hshots)
-        j2.set_batch(B)
+        j2.set_batch(nbatch)
         j2.run()
         im, il, nm = j2.result(normalised=True)
         j2.close()
@@ -487,7 +493,10 @@ def main():
             "config": workload_config(args, B, last_batch),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": (achieved / peak) if achieved else None, "traffic": traffic,
-                         "peak_kind": peak_kind, "kernel": "k_bstep2d_t (fused stencil + time update, pipelined 2D tiles)",
+                         "peak_kind": peak_kind,
+                         "kernel": ("k_onchip2d (wavefields resident on the chip, many steps per "
+                                    "launch; figures per step)" if onchip else
+                                    "k_bstep2d_t (fused stencil + time update, pipelined 2D tiles)"),
                          "avg_launch_ms": (st["step_kernel_ms"] / nl),
                          "algorithmic_bytes_per_launch": algo_per_launch,
                          "launches_timed": st["step_kernel_timed"]},

@@ -2,9 +2,9 @@
 //
 // A shot whose padded grid fits into the shared memory of (a share of) the
 // device runs all its time steps in one cooperative launch.  The grid is cut
-// into tiles, one CTA of 512 threads each; a CTA keeps its tile's four time
-// in shared memory for the whole launch and only exchanges a
-// 4-cell border with its (up to four) neighbours per step.  HBM sees the
+// into tiles, one CTA of 256 threads each; a CTA keeps its tile's four time
+// levels in shared memory for the whole launch and only exchanges a 4-cell
+// border with its (up to four) neighbours per step.  HBM sees the
 // initial and final state, the saved snapshots, the injection terms and the
 // receiver cells; no level is streamed per step.
 //

@@ -194,6 +194,7 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
     }
     if (!fits) tile.stream2d = 1;
   }
+  const int ty0 = tile.ty;
   if (!shots[0].d.g.twoD && tile.stream3d == 2 && tile.ty == StepTile{}.ty) {
     // Planes per work unit of the pipelined 3D kernel (unless tuned): the
     // CTAs take units in turn, so a launch lasts as long as the fullest CTA's
@@ -234,7 +235,10 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
       fits = (g.nmax1 - g.nmin1 + 32) / 32 <= 256 && (g.nmax2 - g.nmin2 + 32) / 32 <= 256 &&
              (g.nmax3 - g.nmin3 + tile.ty) / tile.ty <= 256;
     }
-    if (!fits) tile.stream3d = 1;
+    if (!fits) {
+      tile.stream3d = 1;
+      tile.ty = ty0;
+    }
   }
   const bool t3 = !shots[0].d.g.twoD && tile.stream3d == 2;
   // ---- host-side plans and arena sizes ----
