@@ -710,8 +710,8 @@ __global__ void __launch_bounds__(256, R2_PER_SM) k_brho2d(BatchTables t, int s_
   const float *const pv = S.vel, *const pr = S.rho, *const f1 = S.f[(s + 2) % 5],
               *const f0 = S.f[(s + 1) % 5], *const fm = S.f[s % 5];
   // Divergence times v^2*rho (FDderivatives.f90:642-655) and the point
-  // update, four rows per item: lanes 0-15 of a warp take the 16 row
-  // groups of one column, lanes 16-31 those of the next.
+  // update, four rows per item: lanes 0-7 of a warp take the 8 row groups of
+  // one column, lanes 8-15 those of the next, and so on.
   const int rr = 4 * (tid % R2_G);
 #pragma unroll 1
   for (int h = 0; h < R2_X * R2_G / 256; ++h) {
