@@ -30,9 +30,10 @@
 // ones.  Two CTAs per SM: one computes while the other waits; one CTA of 512
 // threads took 3 % longer, three of 256 or two of 384 (80 registers) 15-25 %,
 // 4 x 4 points per work item 9-15 %.  Time per step against the per-step
-// kernels (one GB300): 201 x 401 modelling 12.4 -> 2.1 us, 301 x 901 RTM
-// 9.2 -> 2.9 us (mean of both passes), four 301 x 901 FWI shots at a time
-// 5.1 us forward, one 751 x 1150 survey shot 4.0 us.
+// kernels (one GB300): 201 x 401 modelling 12.4 -> 2.0 us, 301 x 901 RTM
+// 9.2 -> 2.7 us (mean of both passes).  Forward steps of one, two, three and
+// four 301 x 901 shots at a time take 2.5, 3.2, 4.1 and 4.9 us: 1.5 us of
+// latency (packets, edge lines, barriers) and 0.85 per shot.
 #pragma once
 
 #include "batch.cuh"
