@@ -90,6 +90,25 @@ void deal_tiles(std::vector<int> &tab, const std::vector<T2Shot> &h, int ncta) {
   tab.swap(out);
 }
 
+// Whether a receiver's footprint (half-width h of a sinc gather) may meet a
+// cell that the shared 3D edge launch leaves out because only a line that a
+// later one overwrites elsewhere reaches it: the z padding beside the 4 outer
+// columns or planes of the compute domain, the x padding beside the 4 outer
+// planes.  Receivers are accepted anywhere in the padded grid.
+bool meets_left_out(const Geom &g, const ExtPlan &e, int h) {
+  if (!e.on) return false;
+  if (e.mode == SW_EXT_SIMPLE_AFWI) h = 0;
+  auto pad = [h](int i, int lo, int hi) { return i - h < lo || i + h > hi; };
+  auto outer = [h](int i, int lo, int hi) { return i - h <= lo + 3 || i + h >= hi - 3; };
+  for (int r = 0; r < e.nrec; ++r) {
+    const int i = e.ic[3 * r], j = e.ic[3 * r + 1], k = e.ic[3 * r + 2];
+    const bool kout = outer(k, g.nmin3, g.nmax3);
+    if (pad(i, g.nmin1, g.nmax1) && (kout || outer(j, g.nmin2, g.nmax2))) return true;
+    if (pad(j, g.nmin2, g.nmax2) && kout) return true;
+  }
+  return false;
+}
+
 // 3D FP32 tensor map over a padded field (ld1 x n2p x n3p) with a box of
 // bz rows x bx columns x 1 plane.
 bool encode_field_map3(CUtensorMap *m, const float *base, const Geom &g, int bz, int bx) {
@@ -309,17 +328,18 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
   // The fused 2D edge kernel needs n1, n2 >= 16 in every shot.
   bool fused_edges = !has_3d && !tile.has_surf;
   for (int b = 0; b < nb && fused_edges; ++b) fused_edges = edge_threads_2d(G[b]) > 0;
-  // The 3D edges in one launch (edges3d) leave out padding cells next to the
-  // grid's edges that no receiver within the physical grid gathers from
-  // (half-widths are at most 7); the whole padded field of the last step, if
-  // asked for, still shows them.  Lines are 8 cells and start from 2 more.
+  // The 3D edges in one launch (edges3d) never write the padding cells of
+  // meets_left_out, so no receiver may gather from them; the whole padded
+  // field of the last step, if asked for, still shows them.  Lines are 8
+  // cells and start from 2 more.
   bool edges3 = t3 && !tile.has_surf && !opt.rigid;
   for (int b = 0; b < nb && edges3; ++b) {
     const Geom &g = G[b];
     const int w = std::min({1 - g.nmin1, g.nmax1 - g.nz, 1 - g.nmin2, g.nmax2 - g.nx,
                             1 - g.nmin3, g.nmax3 - g.ny});
     edges3 = w >= 8 && g.nmax1 - g.nmin1 >= 15 && g.nmax2 - g.nmin2 >= 15 &&
-             g.nmax3 - g.nmin3 >= 15 && !shots[b].io.final_u2_host;
+             g.nmax3 - g.nmin3 >= 15 && !shots[b].io.final_u2_host &&
+             !meets_left_out(g, ext[b], shots[b].d.g.lsinc / 2);
   }
   int max_steps = 0;
   for (int b = 0; b < nb; ++b) {

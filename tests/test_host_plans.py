@@ -1,0 +1,55 @@
+"""What the host code decides for a call, on the CPU (tests/fakecuda.py)."""
+import itertools
+
+import numpy as np
+import pytest
+
+from tests.cases import case3d
+from tests.fakecuda import Fake
+
+
+@pytest.fixture()
+def fake():
+    f = Fake()
+    f.reset()
+    return f
+
+
+def _edge_cells(n, shared):
+    """Padded cells (4 around n[0] x n[1] x n[2]) that the 3D edge lines write:
+    all z, x and y lines, or those that the shared launch keeps."""
+    out = np.zeros([m + 8 for m in n], bool)
+    ends = [list(range(0, 8)) + list(range(m, m + 8)) for m in n]    # 8 cells of a line
+    dom = [range(4, m + 4) for m in n]
+    inner = [range(8, m) for m in n]
+    z = (inner[1], inner[2]) if shared else (dom[1], dom[2])
+    x = (dom[0], inner[2]) if shared else (dom[0], dom[2])
+    out[np.ix_(ends[0], *z)] = True
+    out[np.ix_(x[0], ends[1], x[1])] = True
+    out[np.ix_(dom[0], dom[1], ends[2])] = True
+    return out
+
+
+@pytest.mark.parametrize("lsinc", [3, 7, 15])
+def test_receivers_beside_left_out_edge_cells(fake, lsinc):
+    """Every receiver whose footprint meets a padding cell that the shared 3D
+    edge launch leaves out takes the ordered lines; others mostly do not."""
+    g, vel, sou, _, w = case3d(nz=4, nx=5, ny=3, nt=2, ntaper=8)
+    g.lsinc = lsinc
+    n = (g.nz + 16, g.nx + 16, g.ny + 16)
+    missing = _edge_cells(n, False) & ~_edge_cells(n, True)
+    assert missing.any()
+    h = lsinc // 2
+    picks = [sorted({h, h + 1, h + 3, 7, 8, m // 2 + 4, m - 1, m, m + 7 - h - 1, m + 7 - h}
+                    & set(range(h, m + 8 - h))) for m in n]
+    shared = 0
+    with fake.context() as c:
+        for p in itertools.product(*picks):
+            rec = np.array([[(q - 4 - g.ntaper) * 10.0 for q in p]], np.float32)
+            fake.reset()
+            c.modeling(g, vel, sou, w, rec)
+            ordered = bool(fake.kernels("k_bhiggz"))
+            box = tuple(slice(q - h, q + h + 1) for q in p)
+            assert ordered or not missing[box].any(), p
+            shared += not ordered
+    assert shared > 0
