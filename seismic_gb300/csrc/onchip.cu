@@ -124,6 +124,8 @@ bool oc_eligible(const sw_ctx *c, const PhaseShot &p, const RunOpts &opt) {
   if (!d.g.twoD || p.io.rho_pad || d.g.surf_type != 0 || !opt.use_graph || opt.tile.stream2d != 2)
     return false;
   if (d.imaging < SW_IMG_NONE || d.imaging > SW_IMG_BORN) return false;
+  // The adjoint form has no Born source (no driver runs it there).
+  if (d.imaging == SW_IMG_BORN && d.fd_scheme == SW_FD_ADJOINT) return false;
   // A phase that both saves and images may read the slot it writes.
   if (d.extract_wave && d.imaging != SW_IMG_NONE) return false;
   const Geom g = make_geom(d.g);

@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(OC_THREADS, OC_PER_SM) k_onchip2d(OcArgs A) {
     }
   }
   __syncthreads();
-  const bool born = !ADJ && S.imaging == 4 && S.tstep > 0;
+  const bool born = !ADJ && S.imaging == 4 && S.tstep > 0;   // ADJ: oc_eligible
   const bool saves = S.extract_wave || O.bsnap;
   const int tstep = S.tstep, snapi = S.snapi, nz = S.g.nz;
   const int nsave = min(3, snapi);   // steps a snapshot's saving is spread over
