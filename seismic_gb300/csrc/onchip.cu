@@ -117,6 +117,12 @@ cudaError_t launch(const OcArgs &a, int ncta, size_t smem, cudaStream_t s) {
                                      args, smem, s);
 }
 
+bool clear_inbox(sw_ctx *c) {
+  const DBuf &b = c->bufs["oc_inbox"];
+  c->oc_epoch = 0;
+  return cudaMemsetAsync(b.p, 0, b.cap, c->stream) == cudaSuccess;
+}
+
 }  // namespace
 
 bool oc_eligible(const sw_ctx *c, const PhaseShot &p, const RunOpts &opt) {
@@ -377,14 +383,9 @@ bool oc_plan(sw_ctx *c, const std::vector<PhaseShot> &shots, const std::vector<G
   }
   // Packets carry epochs that grow over the context's launches, so what an
   // earlier launch left in the inbox is never taken for a new packet; a new
-  // buffer (or an epoch about to wrap) starts from zero.
-  long long total = 0;
-  for (auto &g : R.groups) total += g.steps + 1;
-  if (c->bufs["oc_inbox"].cap != had || (long long)c->oc_epoch + total >= 0xffffffffLL) {
-    if (cudaMemsetAsync(R.d_inbox, 0, c->bufs["oc_inbox"].cap, c->stream) != cudaSuccess)
-      return false;
-    c->oc_epoch = 0;
-  }
+  // buffer starts from zero, and so does a launch before which the epochs
+  // would wrap (oc_run).
+  if (c->bufs["oc_inbox"].cap != had && !clear_inbox(c)) return false;
   return true;
 }
 
@@ -452,8 +453,11 @@ int oc_run(sw_ctx *c, const std::vector<ShotDev> &hs, const ShotDev *dshots, OcR
       for (int s0 = 0; s0 < g.steps; s0 += g.chunk) {
         a.s0 = s0;
         a.s1 = std::min(s0 + g.chunk, g.steps);
+        const unsigned used = (unsigned)(a.s1 - a.s0) + 1;
+        if (c->oc_epoch > 0xffffffffu - used && !clear_inbox(c))
+          return cuda_fail(c, cudaGetLastError(), "on-chip inbox");
         a.epoch0 = c->oc_epoch;
-        c->oc_epoch += (unsigned)(a.s1 - a.s0) + 1;
+        c->oc_epoch += used;
         for (int b : g.members) {
           const int ns = std::min(a.s1, hs[b].nsteps) - s0;
           if (ns <= 0 || !R.shot[b].nent) continue;

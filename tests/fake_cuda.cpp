@@ -6,7 +6,7 @@
 // k_onchip2d is checked as it is launched: its CTAs take a border packet when
 // it carries the epoch of the step, so no packet that is in the inbox before
 // the launch may carry an epoch of the launch.  The fake then leaves the
-// launch's own epochs there.
+// launch's own epochs in half of it (a launch does not use every slot).
 #include <cuda_runtime.h>
 #include <cuda.h>
 
@@ -70,7 +70,7 @@ cudaError_t launch(const void *f, dim3 g, dim3 b, void **args, bool coop) {
       const uint64_t e = A.inbox[q];
       if ((e >= first && e <= end) || (end >> 32 && e <= (end & 0xffffffffu))) ++stale;
     }
-    for (size_t q = 1; q < words; q += 2) A.inbox[q] = (uint32_t)(end - (q / 2) % 2);
+    for (size_t q = 1; q < words; q += 4) A.inbox[q] = (uint32_t)(end - (q / 4) % 2);
   }
   launches.push_back({n, g, b, coop});
   return cudaSuccess;

@@ -4,7 +4,7 @@ import itertools
 import numpy as np
 import pytest
 
-from tests.cases import case3d
+from tests.cases import case2d, case3d
 from tests.fakecuda import Fake
 
 
@@ -53,3 +53,22 @@ def test_receivers_beside_left_out_edge_cells(fake, lsinc):
             assert ordered or not missing[box].any(), p
             shared += not ordered
     assert shared > 0
+
+
+def test_onchip_epochs_do_not_wrap(fake):
+    """A run of several on-chip launches that starts anywhere near the end of
+    the 32-bit epochs never finds a packet of its own epochs in the inbox."""
+    g, vel, sou, rec, w = case2d(nz=150, nx=200, nt=260, snapi=1)
+    data = np.zeros((len(rec), g.nt), np.float32)
+    fake.reset(70 << 20)      # scratch for about 50 steps per launch
+    with fake.context() as c:
+        c.rtm(g, vel, sou, w, rec, data)
+        n = len(fake.kernels("k_onchip2d"))
+        first = fake.lib.fake_epoch(c.h)
+        c.rtm(g, vel, sou, w, rec, data)
+        used = fake.lib.fake_epoch(c.h) - first
+        assert n > 3 and used > 2 * g.nt
+        for left in [*range(0, 12), *range(used - 12, used + 3), 70, 71, 72, 261, 262, 263]:
+            fake.lib.fake_set_epoch(c.h, 2 ** 32 - 1 - left)
+            c.rtm(g, vel, sou, w, rec, data)
+            assert fake.lib.fake_stale() == 0, left
