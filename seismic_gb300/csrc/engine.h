@@ -39,6 +39,7 @@ struct sw_ctx {
   sw_stats stats{};
   RunOpts run_opts;
   unsigned oc_epoch = 0;   // last packet epoch of the on-chip kernel's inbox
+  bool oc_zeroed = false;  // the inbox holds zeros or packets up to oc_epoch
   std::vector<std::pair<void *, size_t>> touch;   // see TouchWhileBusy
 };
 

@@ -120,7 +120,7 @@ cudaError_t launch(const OcArgs &a, int ncta, size_t smem, cudaStream_t s) {
 bool clear_inbox(sw_ctx *c) {
   const DBuf &b = c->bufs["oc_inbox"];
   c->oc_epoch = 0;
-  return cudaMemsetAsync(b.p, 0, b.cap, c->stream) == cudaSuccess;
+  return c->oc_zeroed = cudaMemsetAsync(b.p, 0, b.cap, c->stream) == cudaSuccess;
 }
 
 }  // namespace
@@ -370,9 +370,15 @@ bool oc_plan(sw_ctx *c, const std::vector<PhaseShot> &shots, const std::vector<G
   }
   int st = SW_OK;
   const std::string keep = c->err;
+  // Packets carry epochs that grow over the context's launches, so what an
+  // earlier launch left in the inbox is never taken for a new packet; a new
+  // buffer starts from zero, and so does a launch before which the epochs
+  // would wrap (oc_run).
   const size_t had = c->bufs["oc_inbox"].cap;
-  R.d_scratch = (char *)dbuf(c, "oc_scratch", R.scratch, &st);
   R.d_inbox = dbuf(c, "oc_inbox", R.inbox, &st);
+  if (c->bufs["oc_inbox"].cap != had) c->oc_zeroed = false;
+  if (R.d_inbox && !c->oc_zeroed && !clear_inbox(c)) return false;
+  R.d_scratch = (char *)dbuf(c, "oc_scratch", R.scratch, &st);
   R.d_tiles = dbuf(c, "oc_tiles", R.tiles.size() * sizeof(OcTile), &st);
   R.d_cells = dbuf(c, "oc_cells", R.cells.size() * sizeof(int), &st);
   R.d_idx = dbuf(c, "oc_idx", R.idx.size() * sizeof(int), &st);
@@ -381,11 +387,6 @@ bool oc_plan(sw_ctx *c, const std::vector<PhaseShot> &shots, const std::vector<G
     c->err = keep;
     return false;
   }
-  // Packets carry epochs that grow over the context's launches, so what an
-  // earlier launch left in the inbox is never taken for a new packet; a new
-  // buffer starts from zero, and so does a launch before which the epochs
-  // would wrap (oc_run).
-  if (c->bufs["oc_inbox"].cap != had && !clear_inbox(c)) return false;
   return true;
 }
 

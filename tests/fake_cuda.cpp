@@ -1,6 +1,6 @@
 // A CUDA runtime without a device, for tests of libswave's host code on the
-// CPU: device memory is host memory (filled with 0xff when allocated), copies
-// and sets are done at once, kernels are recorded and do nothing, and the test
+// CPU: device memory is host memory (small numbers when allocated), copies and
+// sets are done at once, kernels are recorded and do nothing, and the test
 // decides what fails.  Linked with libswave's own objects in place of cudart.
 //
 // k_onchip2d is checked as it is launched: its CTAs take a border packet when
@@ -158,7 +158,7 @@ cudaError_t cudaMalloc(void **p, size_t n) {
   if (fail_alloc >= 0) --fail_alloc;
   if (refuse || used + n > limit) return ret(cudaErrorMemoryAllocation);
   *p = std::aligned_alloc(256, (n + 255) / 256 * 256);
-  std::memset(*p, 0xff, n);
+  for (size_t q = 0; q < n / 4; ++q) ((uint32_t *)*p)[q] = q % 1021;
   mem[*p] = n;
   used += n;
   return cudaSuccess;

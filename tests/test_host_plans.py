@@ -4,6 +4,7 @@ import itertools
 import numpy as np
 import pytest
 
+import seismic_gb300 as sw
 from tests.cases import case2d, case3d
 from tests.fakecuda import Fake
 
@@ -72,3 +73,24 @@ def test_onchip_epochs_do_not_wrap(fake):
             fake.lib.fake_set_epoch(c.h, 2 ** 32 - 1 - left)
             c.rtm(g, vel, sou, w, rec, data)
             assert fake.lib.fake_stale() == 0, left
+
+
+def test_onchip_inbox_after_a_refused_allocation(fake):
+    """Whichever allocation of a call is refused, the next call does not take
+    what its memory held before for packets."""
+    small = case2d(nz=60, nx=80, nt=40)
+    g, vel, sou, rec, w = case2d(nz=200, nx=330, nt=90)
+    for k in range(40):
+        fake.reset()
+        with fake.context() as c:
+            c.modeling(*small[:3], small[4], small[3])
+            n = len(fake.kernels("k_onchip2d"))
+            fake.lib.fake_fail_alloc(k)
+            try:
+                c.modeling(g, vel, sou, w, rec)
+            except sw.SwaveError as e:
+                assert e.code == sw.SW_OOM_ADMISSION
+            fake.lib.fake_fail_alloc(-1)
+            c.modeling(g, vel, sou, w, rec)
+            assert len(fake.kernels("k_onchip2d")) > n
+            assert fake.lib.fake_stale() == 0, k
