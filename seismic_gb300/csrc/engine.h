@@ -22,6 +22,7 @@ struct RunOpts {
   int chunk = 16;       // steps per captured graph
   bool use_graph = true;
   bool rigid = false;   // skip the Higdon boundary (exact-adjoint mode)
+  bool onchip = true;   // 2D shots that fit run on the chip
   swave::StepTile tile; // fused-step tile shape
   // Return once the phase is queued: the kernels record errors in the
   // context's "run_err" flag, which the caller zeroes before and reads after
@@ -40,6 +41,7 @@ struct sw_ctx {
   RunOpts run_opts;
   unsigned oc_epoch = 0;   // last packet epoch of the on-chip kernel's inbox
   bool oc_zeroed = false;  // the inbox holds zeros or packets up to oc_epoch
+  int oc_resident[4] = {-1, -1, -1, -1};   // CTAs of the on-chip kernel's forms; -1: not asked
   std::vector<std::pair<void *, size_t>> touch;   // see TouchWhileBusy
 };
 
@@ -157,7 +159,7 @@ bool oc_eligible(const sw_ctx *c, const PhaseShot &p, const RunOpts &opt);
 bool oc_plan(sw_ctx *c, const std::vector<PhaseShot> &shots, const std::vector<Geom> &G,
              const std::vector<InjPlan> &inj, const std::vector<ExtPlan> &ext, OcRun &R);
 int oc_run(sw_ctx *c, const std::vector<ShotDev> &hs, const ShotDev *dshots, OcRun &R, bool rigid,
-           int *derr, uint64_t *launches);
+           int *derr, uint64_t *launches, bool *refused);
 
 int fail(sw_ctx *c, int code, const char *fmt, ...);
 

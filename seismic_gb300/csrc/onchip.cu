@@ -97,24 +97,33 @@ int num_sms(int dev) {
   return n;
 }
 
-template <bool ADJ, bool VSM>
-cudaError_t launch(const OcArgs &a, int ncta, size_t smem, cudaStream_t s) {
-  // The shared-memory opt-in is a per-device function attribute.
-  static unsigned long long attr_set = 0;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev >= 64 || !(attr_set & (1ull << dev))) {
-    e = cudaFuncSetAttribute(k_onchip2d<ADJ, VSM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kSmemLimit);
-    if (e != cudaSuccess) return e;
-    if (dev < 64) attr_set |= 1ull << dev;
+// What the kernel keeps in static shared memory beside a CTA's kSmemLimit (and
+// the 1 KB that the system takes of each CTA's share).
+static_assert(kSmemLimit + sizeof(ShotDev) + 40 * sizeof(int) + 1024 <= 228 * 1024 / OC_PER_SM,
+              "OC_PER_SM CTAs of k_onchip2d no longer fit on an SM");
+
+const void *kernel(bool adj, bool vsm) {
+  return adj ? (vsm ? (const void *)k_onchip2d<true, true> : (const void *)k_onchip2d<true, false>)
+             : (vsm ? (const void *)k_onchip2d<false, true> : (const void *)k_onchip2d<false, false>);
+}
+
+// CTAs of a form that are resident together on the context's device, asked
+// once per context (with the shared-memory opt-in); 0 if it cannot be told.
+int resident(sw_ctx *c, bool adj, bool vsm) {
+  int &n = c->oc_resident[2 * adj + vsm];
+  if (n < 0) {
+    int per = 0;
+    const void *k = kernel(adj, vsm);
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, OC_THREADS, kSmemLimit) !=
+            cudaSuccess) {
+      cudaGetLastError();
+      per = 0;
+    }
+    n = per * num_sms(c->device);
   }
-  // Cooperative: the CTAs wait for one another, so all must be resident.
-  OcArgs arg = a;
-  void *args[] = {&arg};
-  return cudaLaunchCooperativeKernel((const void *)k_onchip2d<ADJ, VSM>, dim3(ncta), dim3(OC_THREADS),
-                                     args, smem, s);
+  return n;
 }
 
 bool clear_inbox(sw_ctx *c) {
@@ -127,7 +136,8 @@ bool clear_inbox(sw_ctx *c) {
 
 bool oc_eligible(const sw_ctx *c, const PhaseShot &p, const RunOpts &opt) {
   const sw_prop_desc &d = p.d;
-  if (!d.g.twoD || p.io.rho_pad || d.g.surf_type != 0 || !opt.use_graph || opt.tile.stream2d != 2)
+  if (!d.g.twoD || p.io.rho_pad || d.g.surf_type != 0 || !opt.use_graph ||
+      opt.tile.stream2d != 2 || !opt.onchip)
     return false;
   if (d.imaging < SW_IMG_NONE || d.imaging > SW_IMG_BORN) return false;
   // The adjoint form has no Born source (no driver runs it there).
@@ -141,8 +151,8 @@ bool oc_eligible(const sw_ctx *c, const PhaseShot &p, const RunOpts &opt) {
 }
 
 // Cuts the shots into launches and carves their plans; false (without an
-// error) when the scratch does not fit, and the caller takes the per-step
-// kernels.
+// error) when the scratch does not fit or the CTAs of a launch would not all
+// be resident, and the caller takes the per-step kernels.
 bool oc_plan(sw_ctx *c, const std::vector<PhaseShot> &shots, const std::vector<Geom> &G,
              const std::vector<InjPlan> &inj, const std::vector<ExtPlan> &ext, OcRun &R) {
   const int nb = (int)shots.size(), nsm = OC_PER_SM * num_sms(c->device);
@@ -350,6 +360,7 @@ bool oc_plan(sw_ctx *c, const std::vector<PhaseShot> &shots, const std::vector<G
         g.vsm = k & 1;
         g.pad = k & 2;
       }
+    if (g.ncta > resident(c, g.adj, g.vsm)) return false;
     size_t freeb = 0, totalb = 0;
     if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) return false;
     size_t held = 0;
@@ -390,9 +401,11 @@ bool oc_plan(sw_ctx *c, const std::vector<PhaseShot> &shots, const std::vector<G
   return true;
 }
 
-// Runs the planned launches on the context's stream.
+// Runs the planned launches on the context's stream.  *refused: the device
+// would not take the first of them (a share of it is held elsewhere) and
+// nothing has run but the injection terms.
 int oc_run(sw_ctx *c, const std::vector<ShotDev> &hs, const ShotDev *dshots, OcRun &R, bool rigid,
-           int *derr, uint64_t *launches) {
+           int *derr, uint64_t *launches, bool *refused) {
   cudaStream_t s = c->stream;
   cudaError_t e;
   const int nb = (int)hs.size();
@@ -440,6 +453,7 @@ int oc_run(sw_ctx *c, const std::vector<ShotDev> &hs, const ShotDev *dshots, OcR
     SW_CK(cudaEventCreate(&ev[1]));
   }
   int st = SW_OK;
+  bool ran = false;
   auto run = [&]() -> int {
     for (auto &g : R.groups) {
       OcArgs a;
@@ -467,11 +481,17 @@ int oc_run(sw_ctx *c, const std::vector<ShotDev> &hs, const ShotDev *dshots, OcR
           ++*launches;
         }
         if (c->profiling) SW_CK(cudaEventRecord(ev[0], s));
-        e = g.adj ? (g.vsm ? launch<true, true>(a, g.ncta, g.smem, s)
-                           : launch<true, false>(a, g.ncta, g.smem, s))
-                  : (g.vsm ? launch<false, true>(a, g.ncta, g.smem, s)
-                           : launch<false, false>(a, g.ncta, g.smem, s));
+        // Cooperative: the CTAs wait for one another, so all must be resident.
+        void *args[] = {&a};
+        e = cudaLaunchCooperativeKernel(kernel(g.adj, g.vsm), dim3(g.ncta), dim3(OC_THREADS), args,
+                                        g.smem, s);
+        if (!ran && (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported)) {
+          cudaGetLastError();
+          *refused = true;
+          return SW_OK;
+        }
         if (e != cudaSuccess) return cuda_fail(c, e, "on-chip propagation");
+        ran = true;
         ++*launches;
         if (c->profiling) {
           SW_CK(cudaEventRecord(ev[1], s));

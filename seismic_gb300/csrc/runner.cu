@@ -820,7 +820,13 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
   };
   uint64_t launches = 0;
   if (oc) {
-    if ((st = oc_run(c, hs, dshots, ocr, opt.rigid, derr, &launches))) return st;
+    bool refused = false;
+    if ((st = oc_run(c, hs, dshots, ocr, opt.rigid, derr, &launches, &refused))) return st;
+    if (refused) {
+      RunOpts per_step = opt;
+      per_step.onchip = false;
+      return run_phases(c, shots, per_step);
+    }
     if (prof) {
       c->stats.step_kernel_timed += (uint64_t)max_steps;
       for (int q = 0; q < max_steps; ++q) c->stats.step_bytes += step_bytes_at(q);

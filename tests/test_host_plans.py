@@ -94,3 +94,35 @@ def test_onchip_inbox_after_a_refused_allocation(fake):
             c.modeling(g, vel, sou, w, rec)
             assert len(fake.kernels("k_onchip2d")) > n
             assert fake.lib.fake_stale() == 0, k
+
+
+CUDA_ERROR_COOPERATIVE_LAUNCH_TOO_LARGE, CUDA_ERROR_LAUNCH_FAILURE = 720, 719
+
+
+@pytest.mark.parametrize("how", ["residency", "launch"])
+def test_onchip_refused_by_the_device(fake, how):
+    """Where the CTAs of an on-chip launch are not all resident, or the device
+    does not take the launch, the call runs through the per-step kernels;
+    shots small enough for the smaller residency stay on the chip, and other
+    errors are returned."""
+    g, vel, sou, rec, w = case2d(nz=300, nx=600, nt=60)
+    data = np.zeros((len(rec), g.nt), np.float32)
+    small = case2d(nz=60, nx=80, nt=40)
+    with fake.context() as c:
+        c.rtm(g, vel, sou, w, rec, data)
+        assert fake.kernels("k_onchip2d") and not fake.kernels("k_bstep2d_t")
+    fake.reset()
+    if how == "residency":
+        fake.lib.fake_blocks_per_sm(1)
+    else:
+        fake.lib.fake_coop_error(CUDA_ERROR_COOPERATIVE_LAUNCH_TOO_LARGE)
+    with fake.context() as c:
+        c.rtm(g, vel, sou, w, rec, data)
+        assert not fake.kernels("k_onchip2d") and fake.kernels("k_bstep2d_t")
+        c.modeling(*small[:3], small[4], small[3])
+        assert bool(fake.kernels("k_onchip2d")) == (how == "residency")
+    if how == "launch":
+        fake.lib.fake_coop_error(CUDA_ERROR_LAUNCH_FAILURE)
+        with fake.context() as c, pytest.raises(sw.SwaveError) as e:
+            c.rtm(g, vel, sou, w, rec, data)
+        assert e.value.code == sw.SW_CUDA_ERR
