@@ -316,11 +316,15 @@ cudaError_t launch_rho_delp(const Geom &g, const float *rho_pad, float *delp, fl
 // The first two outputs of every section stay zero, as the reference's
 // never-written work samples do.
 // ---------------------------------------------------------------------------
+// A block of k_bp_pad and k_bp_cut takes 32 traces x 32 samples, trace blocks
+// fastest in one grid dimension: the others hold 65535 blocks, fewer than
+// long records or many traces need.
 __global__ void __launch_bounds__(256) k_bp_pad(int ntr, int nt, int npad, const float *lead,
                                                 const float *trail, const float *__restrict__ in,
                                                 float *__restrict__ D) {
   __shared__ float tile[32][33];
-  const int n = nt + 2 * npad, t0 = 32 * blockIdx.x, i0 = 32 * blockIdx.y;
+  const int n = nt + 2 * npad, gx = (ntr + 31) / 32;
+  const int t0 = 32 * (blockIdx.x % gx), i0 = 32 * (blockIdx.x / gx);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int r = w; r < 32; r += 8) {
     const int t = t0 + r, i = i0 + lane;
@@ -338,7 +342,7 @@ __global__ void __launch_bounds__(256) k_bp_cut(int ntr, int nt, int npad,
                                                 const float *__restrict__ D,
                                                 float *__restrict__ out) {
   __shared__ float tile[32][33];
-  const int t0 = 32 * blockIdx.x, i0 = 32 * blockIdx.y;
+  const int gx = (ntr + 31) / 32, t0 = 32 * (blockIdx.x % gx), i0 = 32 * (blockIdx.x / gx);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int r = w; r < 32; r += 8)
     if (t0 + lane < ntr && i0 + r < nt)
@@ -426,13 +430,14 @@ cudaError_t launch_bandpass(int ntr, int nt, int npad, int phase, int nlo, const
                             int nhi, const float *chi, const float *lead, const float *trail,
                             const float *in, float *out, float *D, cudaStream_t s,
                             int *nlaunch) {
-  const int n = nt + 2 * npad, gx = (ntr + 31) / 32;
-  k_bp_pad<<<dim3(gx, (n + 31) / 32), 256, 0, s>>>(ntr, nt, npad, lead, trail, in, D);
+  const int n = nt + 2 * npad;
+  const unsigned gx = (ntr + 31) / 32;
+  k_bp_pad<<<gx * ((n + 31) / 32), 256, 0, s>>>(ntr, nt, npad, lead, trail, in, D);
   launch_bp_sections(ntr, n, 0, nlo, clo, D, s, nlaunch);
   if (phase == 0) launch_bp_sections(ntr, n, 1, nlo, clo, D, s, nlaunch);
   launch_bp_sections(ntr, n, 0, nhi, chi, D, s, nlaunch);
   if (phase == 0) launch_bp_sections(ntr, n, 1, nhi, chi, D, s, nlaunch);
-  k_bp_cut<<<dim3(gx, (nt + 31) / 32), 256, 0, s>>>(ntr, nt, npad, D, out);
+  k_bp_cut<<<gx * ((nt + 31) / 32), 256, 0, s>>>(ntr, nt, npad, D, out);
   *nlaunch += 2;
   return cudaGetLastError();
 }

@@ -126,3 +126,10 @@ def test_onchip_refused_by_the_device(fake, how):
         with fake.context() as c, pytest.raises(sw.SwaveError) as e:
             c.rtm(g, vel, sou, w, rec, data)
         assert e.value.code == sw.SW_CUDA_ERR
+
+
+@pytest.mark.parametrize("ntr,nt", [(1, 2), (1, 2_097_153), (3, 2_200_000), (2_097_185, 3)])
+def test_bandpass_takes_every_size(fake, ntr, nt):
+    with fake.context() as c:
+        c.bandpass(np.ones((ntr, nt), np.float32), 2e-3, flo=5.0, fhi=90.0)
+    assert len(fake.kernels("k_bp_pad")) == len(fake.kernels("k_bp_cut")) == 1
