@@ -874,15 +874,16 @@ int ensure_images(sw_cnn *n, size_t npix) {
   for (int c : n->ch) cmax = std::max(cmax, cstore(c));
   n->a.assign(n->nl, nullptr);
   for (int l = 0; l < n->nl && ok; ++l)
-    ok = ck(cudaMalloc(&n->a[l], npix * cstore(n->ch[l]) * sizeof(__nv_bfloat16)));
-  ok = ok && ck(cudaMalloc(&n->dz[0], npix * cmax * sizeof(__nv_bfloat16))) &&
-       ck(cudaMalloc(&n->dz[1], npix * cmax * sizeof(__nv_bfloat16))) &&
-       ck(cudaMalloc(&n->out32, npix * sizeof(float))) &&
-       ck(cudaMalloc(&n->in32, npix * n->ch[0] * sizeof(float))) &&
-       ck(cudaMalloc(&n->tgt, npix * sizeof(float))) &&
-       ck(cudaMalloc(&n->part, (size_t)n->nl * num_sms(n->ctx->device) * part_floats(n->taps) *
-                               sizeof(float))) &&
-       ck(cudaMalloc(&n->lpart, 1024 * sizeof(double)));
+    ok = ck(dev_malloc(n->ctx, &n->a[l], npix * cstore(n->ch[l]) * sizeof(__nv_bfloat16)));
+  ok = ok && ck(dev_malloc(n->ctx, &n->dz[0], npix * cmax * sizeof(__nv_bfloat16))) &&
+       ck(dev_malloc(n->ctx, &n->dz[1], npix * cmax * sizeof(__nv_bfloat16))) &&
+       ck(dev_malloc(n->ctx, &n->out32, npix * sizeof(float))) &&
+       ck(dev_malloc(n->ctx, &n->in32, npix * n->ch[0] * sizeof(float))) &&
+       ck(dev_malloc(n->ctx, &n->tgt, npix * sizeof(float))) &&
+       ck(dev_malloc(n->ctx, &n->part,
+                     (size_t)n->nl * num_sms(n->ctx->device) * part_floats(n->taps) *
+                         sizeof(float))) &&
+       ck(dev_malloc(n->ctx, &n->lpart, 1024 * sizeof(double)));
   if (!ok) {
     cudaGetLastError();
     free_images(n);
@@ -1088,15 +1089,15 @@ int create_net(sw_ctx *c, int nlayers, const int *channels, uint64_t seed, int t
     for (int q = 0; q < Cout * taps * Cin; ++q) h[n->woff[l] + q] = nd(rng);
   }
   auto ck = [](cudaError_t e) { return e == cudaSuccess; };
-  bool ok = ck(cudaMalloc(&n->w, n->nw * 4)) && ck(cudaMalloc(&n->g, n->nw * 4)) &&
-            ck(cudaMalloc(&n->m, n->nw * 4)) && ck(cudaMalloc(&n->v, n->nw * 4)) &&
-            ck(cudaMalloc(&n->err, sizeof(int)));
+  bool ok = ck(dev_malloc(c, &n->w, n->nw * 4)) && ck(dev_malloc(c, &n->g, n->nw * 4)) &&
+            ck(dev_malloc(c, &n->m, n->nw * 4)) && ck(dev_malloc(c, &n->v, n->nw * 4)) &&
+            ck(dev_malloc(c, &n->err, sizeof(int)));
   n->wf.assign(nlayers, nullptr);
   n->wb.assign(nlayers, nullptr);
   for (int l = 0; l < nlayers && ok; ++l) {
     const int Cin = n->ch[l], Cout = n->ch[l + 1];
-    ok = ck(cudaMalloc(&n->wf[l], (size_t)r16(Cout) * r16(taps * cstore(Cin)) * 2)) &&
-         ck(cudaMalloc(&n->wb[l], (size_t)r16(Cin) * r16(taps * cstore(Cout)) * 2));
+    ok = ck(dev_malloc(c, &n->wf[l], (size_t)r16(Cout) * r16(taps * cstore(Cin)) * 2)) &&
+         ck(dev_malloc(c, &n->wb[l], (size_t)r16(Cin) * r16(taps * cstore(Cout)) * 2));
   }
   ok = ok && ck(cudaMemcpy(n->w, h.data(), n->nw * 4, cudaMemcpyHostToDevice)) &&
        ck(cudaMemset(n->m, 0, n->nw * 4)) && ck(cudaMemset(n->v, 0, n->nw * 4)) &&

@@ -127,6 +127,34 @@ int cuda_fail(sw_ctx *c, cudaError_t e, const char *what) {
 }
 
 // Grow-only named device buffers owned by the context.
+static bool oc_name(const std::string &name) { return name.compare(0, 3, "oc_") == 0; }
+
+size_t oc_held(const sw_ctx *c) {
+  size_t n = 0;
+  for (auto &kv : c->bufs)
+    if (oc_name(kv.first)) n += kv.second.cap;
+  return n;
+}
+
+bool oc_release(sw_ctx *c) {
+  if (c->oc_use || oc_held(c) == 0) return false;
+  for (auto &kv : c->bufs)
+    if (oc_name(kv.first)) {
+      cudaFree(kv.second.p);
+      kv.second = DBuf();
+    }
+  return true;
+}
+
+cudaError_t dev_malloc(sw_ctx *c, void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && oc_release(c)) {
+    cudaGetLastError();
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+
 void *dbuf(sw_ctx *c, const std::string &name, size_t bytes, int *st, size_t slack) {
   if (bytes == 0) bytes = 16;
   DBuf &b = c->bufs[name];
@@ -135,10 +163,12 @@ void *dbuf(sw_ctx *c, const std::string &name, size_t bytes, int *st, size_t sla
     b.p = nullptr;
     b.cap = 0;
     cudaError_t e = cudaMalloc(&b.p, bytes + slack);
-    if (e == cudaErrorMemoryAllocation && slack > 0) {
+    // The on-chip plan's own buffers do not push one another out.
+    const bool own = oc_name(name);
+    if (e == cudaErrorMemoryAllocation && (slack > 0 || !own)) {
       cudaGetLastError();
       slack = 0;
-      e = cudaMalloc(&b.p, bytes);
+      e = own ? cudaMalloc(&b.p, bytes) : dev_malloc(c, &b.p, bytes);
     }
     if (e != cudaSuccess) {
       cudaGetLastError();

@@ -41,6 +41,7 @@ struct sw_ctx {
   RunOpts run_opts;
   unsigned oc_epoch = 0;   // last packet epoch of the on-chip kernel's inbox
   bool oc_zeroed = false;  // the inbox holds zeros or packets up to oc_epoch
+  bool oc_use = false;     // a phase being queued uses the on-chip plan's buffers
   int oc_resident[4] = {-1, -1, -1, -1};   // CTAs of the on-chip kernel's forms; -1: not asked
   std::vector<std::pair<void *, size_t>> touch;   // see TouchWhileBusy
 };
@@ -160,6 +161,19 @@ bool oc_plan(sw_ctx *c, const std::vector<PhaseShot> &shots, const std::vector<G
              const std::vector<InjPlan> &inj, const std::vector<ExtPlan> &ext, OcRun &R);
 int oc_run(sw_ctx *c, const std::vector<ShotDev> &hs, const ShotDev *dshots, OcRun &R, bool rigid,
            int *derr, uint64_t *launches, bool *refused);
+
+// The on-chip plan's buffers ("oc_...") stay with the context between calls.
+// They are given back when memory runs out (dev_malloc, and dbuf through it),
+// so that what fits beside the per-step kernels fits beside these: frees them
+// unless a phase being queued uses them (cudaFree waits for queued ones), and
+// returns whether there was something to free.
+bool oc_release(sw_ctx *c);
+size_t oc_held(const sw_ctx *c);   // bytes
+cudaError_t dev_malloc(sw_ctx *c, void **p, size_t bytes);
+template <class T>
+cudaError_t dev_malloc(sw_ctx *c, T **p, size_t bytes) {
+  return dev_malloc(c, reinterpret_cast<void **>(p), bytes);
+}
 
 int fail(sw_ctx *c, int code, const char *fmt, ...);
 

@@ -475,7 +475,7 @@ int fct_gdt_batched(sw_ctx *c, const sw_fwi_desc &d, int ntype, const float *vel
     size_t held = 0;
     auto it = c->bufs.find("fwi_arena");
     if (it != c->bufs.end()) held = it->second.cap;
-    const double budget = (double)(freeb + held) * 0.85;
+    const double budget = (double)(freeb + held + oc_held(c)) * 0.85;
     int end = next;
     size_t need = 0, arena = 0;
     while (end < nshot && end - next < kFwiBatch) {
@@ -1129,13 +1129,14 @@ int sw_lbfgs_create(sw_ctx *c, int n, int m, double xmin, double xmax, const flo
   L->rho.assign(m + 1, 0.0);
   L->alpha.assign(m + 1, 0.0);
   const size_t nb = (size_t)n * sizeof(double);
-  bool ok = cudaMalloc(&L->mask, (size_t)n * sizeof(float)) == cudaSuccess &&
-            cudaMalloc(&L->xinit, nb) == cudaSuccess &&
-            cudaMalloc(&L->S, nb * m) == cudaSuccess && cudaMalloc(&L->Y, nb * m) == cudaSuccess &&
-            cudaMalloc(&L->w0, nb) == cudaSuccess && cudaMalloc(&L->wa, nb) == cudaSuccess &&
-            cudaMalloc(&L->x, nb) == cudaSuccess && cudaMalloc(&L->g, nb) == cudaSuccess &&
-            cudaMalloc(&L->part, kRedBlocks * sizeof(double)) == cudaSuccess &&
-            cudaMalloc(&L->res, sizeof(double)) == cudaSuccess;
+  bool ok = dev_malloc(c, &L->mask, (size_t)n * sizeof(float)) == cudaSuccess &&
+            dev_malloc(c, &L->xinit, nb) == cudaSuccess &&
+            dev_malloc(c, &L->S, nb * m) == cudaSuccess &&
+            dev_malloc(c, &L->Y, nb * m) == cudaSuccess &&
+            dev_malloc(c, &L->w0, nb) == cudaSuccess && dev_malloc(c, &L->wa, nb) == cudaSuccess &&
+            dev_malloc(c, &L->x, nb) == cudaSuccess && dev_malloc(c, &L->g, nb) == cudaSuccess &&
+            dev_malloc(c, &L->part, kRedBlocks * sizeof(double)) == cudaSuccess &&
+            dev_malloc(c, &L->res, sizeof(double)) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
     free_lbfgs(L);
@@ -1306,13 +1307,14 @@ int sw_lbfgs_oc_step(sw_ctx *c, const sw_lbfgs_oc_desc *d, double *xh, double f,
   L->alpha.assign(m + 1, 0.0);
   const size_t nb = (size_t)n * sizeof(double);
   const int np = d->nparam;
-  bool ok = cudaMalloc(&L->S, nb * m) == cudaSuccess && cudaMalloc(&L->Y, nb * m) == cudaSuccess &&
-            cudaMalloc(&L->w0, nb) == cudaSuccess && cudaMalloc(&L->wa, nb) == cudaSuccess &&
-            cudaMalloc(&L->x, nb) == cudaSuccess && cudaMalloc(&L->g, nb) == cudaSuccess &&
-            cudaMalloc(&L->part, kRedBlocks * sizeof(double)) == cudaSuccess &&
-            cudaMalloc(&L->res, sizeof(double)) == cudaSuccess &&
-            cudaMalloc(&L->pmin, np * sizeof(double)) == cudaSuccess &&
-            cudaMalloc(&L->pmax, np * sizeof(double)) == cudaSuccess;
+  bool ok = dev_malloc(c, &L->S, nb * m) == cudaSuccess &&
+            dev_malloc(c, &L->Y, nb * m) == cudaSuccess &&
+            dev_malloc(c, &L->w0, nb) == cudaSuccess && dev_malloc(c, &L->wa, nb) == cudaSuccess &&
+            dev_malloc(c, &L->x, nb) == cudaSuccess && dev_malloc(c, &L->g, nb) == cudaSuccess &&
+            dev_malloc(c, &L->part, kRedBlocks * sizeof(double)) == cudaSuccess &&
+            dev_malloc(c, &L->res, sizeof(double)) == cudaSuccess &&
+            dev_malloc(c, &L->pmin, np * sizeof(double)) == cudaSuccess &&
+            dev_malloc(c, &L->pmax, np * sizeof(double)) == cudaSuccess;
   auto done = [&](int rc) {
     cudaStreamSynchronize(c->stream);
     free_lbfgs(L);

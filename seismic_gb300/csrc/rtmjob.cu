@@ -231,9 +231,10 @@ int sw_rtm_job_create(sw_ctx *c, const sw_genpar *model, float apx, float apy, c
     return code;
   };
   cudaStream_t s = c->stream;
-  if (cudaMalloc(&j->vel, n * 4) != cudaSuccess || cudaMalloc(&j->image, n * 4) != cudaSuccess ||
-      cudaMalloc(&j->illum, n * 4) != cudaSuccess ||
-      cudaMalloc(&j->wavelet, (size_t)model->nt * 4) != cudaSuccess) {
+  if (dev_malloc(c, &j->vel, n * 4) != cudaSuccess ||
+      dev_malloc(c, &j->image, n * 4) != cudaSuccess ||
+      dev_malloc(c, &j->illum, n * 4) != cudaSuccess ||
+      dev_malloc(c, &j->wavelet, (size_t)model->nt * 4) != cudaSuccess) {
     cudaGetLastError();
     return bail(fail(c, SW_OOM_ADMISSION, "RTM job model buffers do not fit"));
   }
@@ -253,7 +254,7 @@ int sw_rtm_job_create(sw_ctx *c, const sw_genpar *model, float apx, float apy, c
     S.s.rec_coord = S.rec.data();
     const size_t db = (size_t)S.s.nrec * S.s.nt * 4;
     if (S.s.data) {
-      if (cudaMalloc(&S.data, db) != cudaSuccess) {
+      if (dev_malloc(c, &S.data, db) != cudaSuccess) {
         cudaGetLastError();
         return bail(fail(c, SW_OOM_ADMISSION, "RTM job data of shot %d does not fit", i));
       }
@@ -335,7 +336,8 @@ size_t shot_arena_bytes(const sw_genpar &g, int nrec, bool modeling) {
 }
 
 // The admission budget: mem_fraction of the free device memory, the job
-// arena already held counted as free.
+// arena already held (and the on-chip buffers, which make room) counted as
+// free.
 int admission_budget(sw_rtm_job *j, double *budget) {
   sw_ctx *c = j->c;
   size_t freeb = 0, totalb = 0;
@@ -343,7 +345,7 @@ int admission_budget(sw_rtm_job *j, double *budget) {
   size_t held = 0;
   auto it = c->bufs.find("rtm_arena");
   if (it != c->bufs.end()) held = it->second.cap;
-  *budget = (double)(freeb + held) * j->mem_fraction;
+  *budget = (double)(freeb + held + oc_held(c)) * j->mem_fraction;
   return SW_OK;
 }
 

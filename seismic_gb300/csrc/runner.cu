@@ -302,6 +302,17 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
   }
   OcRun ocr;
   oc = oc && oc_plan(c, shots, G, inj, ext, ocr);
+  // The plan's buffers are in use until the phase is queued.
+  struct OcUse {
+    sw_ctx *c;
+    ~OcUse() { c->oc_use = false; }
+  } oc_use{c};
+  c->oc_use = oc;
+  auto per_step = [&]() {   // the phase from its start, off the chip
+    RunOpts o = opt;
+    o.onchip = c->oc_use = false;
+    return run_phases(c, shots, o);
+  };
   const bool t2 = !oc && (tile.stream2d == 2 || tile.stream2d == 3) && shots[0].d.g.twoD;
   bytes += rup(nb * sizeof(ShotDev)) + 9 * rup((nb + 1) * sizeof(int)) + rup(sizeof(int));
   if (t2) {
@@ -318,7 +329,12 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
   bytes += rup(sizeof(int));   // error flags
   // A quarter of headroom when the arena grows: batches of slightly larger
   // windows then reuse it instead of reallocating.
+  const std::string err = c->err;
   char *arena = (char *)dbuf(c, "batch_arena", bytes, &st, bytes / 4);
+  if (!arena && oc && st == SW_OOM_ADMISSION) {   // the plan's buffers make room
+    c->err = err;
+    return per_step();
+  }
   if (!arena) return st;
   char *cur = arena;
   // ---- carve and fill ----
@@ -822,11 +838,7 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
   if (oc) {
     bool refused = false;
     if ((st = oc_run(c, hs, dshots, ocr, opt.rigid, derr, &launches, &refused))) return st;
-    if (refused) {
-      RunOpts per_step = opt;
-      per_step.onchip = false;
-      return run_phases(c, shots, per_step);
-    }
+    if (refused) return per_step();
     if (prof) {
       c->stats.step_kernel_timed += (uint64_t)max_steps;
       for (int q = 0; q < max_steps; ++q) c->stats.step_bytes += step_bytes_at(q);

@@ -1,4 +1,5 @@
 """What the host code decides for a call, on the CPU (tests/fakecuda.py)."""
+import contextlib
 import itertools
 
 import numpy as np
@@ -133,3 +134,70 @@ def test_bandpass_takes_every_size(fake, ntr, nt):
     with fake.context() as c:
         c.bandpass(np.ones((ntr, nt), np.float32), 2e-3, flo=5.0, fhi=90.0)
     assert len(fake.kernels("k_bp_pad")) == len(fake.kernels("k_bp_cut")) == 1
+
+
+def _ok(call):
+    try:
+        call()
+        return True
+    except sw.SwaveError as e:
+        assert e.code == sw.SW_OOM_ADMISSION, e
+        return False
+
+
+def _job(c, g, vel, sou, rec, w, data):
+    job = sw.RTMJob(c, g, vel, w, [{"sou": sou, "rec": rec, "data": data}] * 2)
+    try:
+        job.run()
+    finally:
+        job.close()
+
+
+LATER = {   # what runs on a context that has run a 2D shot on the chip
+    "nothing": lambda c: None,
+    "3d": lambda c: c.modeling(*C3D),
+    "network": lambda c: _network(c),
+    "job": lambda c: _job(c),
+}
+C2D = case2d(nz=160, nx=240, nt=60, nrec=240)
+C3D = [case3d(nz=60, nx=70, ny=64, nt=4)[q] for q in (0, 1, 2, 4, 3)]
+
+
+def _network(c):
+    with contextlib.closing(sw.CNN(c, [2, 16, 1])) as n:
+        n.forward(np.ones((2, 900, 300), np.float32))
+
+
+def _job(c):
+    g, vel, sou, rec, w = C2D
+    d = np.zeros((len(rec), g.nt), np.float32)
+    shots = [{"sou": sou, "rec": rec, "data": d}] * 2
+    with contextlib.closing(sw.RTMJob(c, g, vel, w, shots)) as job:
+        job.run()
+
+
+@pytest.mark.parametrize("later", LATER)
+def test_onchip_buffers_make_room(fake, later):
+    """What fits into the device's memory with the per-step kernels fits with
+    the on-chip path too: a shot by itself, and calls after one whose buffers
+    the context still holds."""
+    g, vel, sou, rec, w = C2D
+    seen = set()
+    for quarter in range(4, 600):
+        ok = []
+        for graph in (0, 1):                 # 0: the per-step kernels
+            fake.reset(quarter << 18)
+            with fake.context() as c:
+                c.set_tuning(use_graph=graph)
+                try:
+                    c.rtm(g, vel, sou, w, rec, np.zeros((len(rec), g.nt), np.float32))
+                    LATER[later](c)
+                    ok.append(True)
+                except sw.SwaveError as e:
+                    assert e.code == sw.SW_OOM_ADMISSION or "cnn create" in str(e), e
+                    ok.append(False)
+        assert ok[1] or not ok[0], quarter
+        seen.add(tuple(ok))
+        if ok == [True, True] and fake.kernels("k_onchip2d"):
+            break
+    assert (False, False) in seen and (True, True) in seen
