@@ -765,9 +765,11 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
       const bool slot = S.tstep > 0 ? cnt <= S.ntsnap : S.ntsnap - cnt + 1 >= 1;
       if (!slot) continue;
       uint64_t per = S.extract_wave ? 4 : 0;
-      if (S.imaging == SW_IMG_RTM || S.imaging == SW_IMG_LSRTM) per += 20;
-      if (S.imaging == SW_IMG_AFWI) per += 28;
-      if (S.imaging == SW_IMG_AFWI_RHO) per += 36;
+      if (!oc) {   // on the chip: k_oc_image, after the timed kernel
+        if (S.imaging == SW_IMG_RTM || S.imaging == SW_IMG_LSRTM) per += 20;
+        if (S.imaging == SW_IMG_AFWI) per += 28;
+        if (S.imaging == SW_IMG_AFWI_RHO) per += 36;
+      }
       if (S.imaging == SW_IMG_BORN) per += 8;
       by += (uint64_t)S.g.nz * S.g.nx * S.g.ny * per;
     }

@@ -201,3 +201,18 @@ def test_onchip_buffers_make_room(fake, later):
         if ok == [True, True] and fake.kernels("k_onchip2d"):
             break
     assert (False, False) in seen and (True, True) in seen
+
+
+def test_profiled_bytes_are_of_the_timed_kernel(fake):
+    """With profiling on, the bytes of an on-chip migration are those of the
+    steps and the saved snapshots; imaging runs in a kernel that is not timed."""
+    g, vel, sou, rec, w = case2d(nz=60, nx=80, nt=60)
+    data = np.zeros((len(rec), g.nt), np.float32)
+    pts = (g.nz + 2 * g.ntaper) * (g.nx + 2 * g.ntaper)
+    steps, saved = 2 * g.nt * pts * 24, (g.nt // g.snapi) * vel.size * 4
+    with fake.context() as c:
+        c.set_profiling(True)
+        c.rtm(g, vel, sou, w, rec, data)
+        st = c.stats()
+        assert fake.kernels("k_oc_image") and st["step_kernel_timed"] == 2 * g.nt
+        assert st["step_bytes"] == steps + saved
