@@ -468,17 +468,22 @@ int sw_lbfgs_oc_step(sw_ctx *ctx, const sw_lbfgs_oc_desc *d, double *x, double f
 
 /* ---- Tuning (no counterpart in the reference: launch shape knobs) -------- */
 typedef struct sw_tuning {
-  int step_kernel;   /* fused step: 0 = 32x8 point tiles, 1 = streaming, 2 = TMA-staged
-                        tiles, 2 CTAs per SM (default), 3 = TMA-staged tiles,
-                        warp-specialised, 4 = two time steps per launch on 64x64 TMA tiles
-                        for 2D batches of up to 32 shots without AFWI / Born
-                        imaging (others run 2); 3D uses streaming for 1 and the
-                        TMA plane pipeline for 2-4 */
+  int step_kernel;   /* 2D: 0 = 32x8 point tiles, 1 = streaming, 2 (default) =
+                        shots that fit run on the chip, many steps per launch
+                        (constant density, no free surface, use_graph != 0),
+                        the others as 5; 3 = TMA-staged tiles,
+                        warp-specialised, 4 = two time steps per launch on
+                        64x64 TMA tiles for batches of up to 32 shots without
+                        AFWI / Born imaging (others run 5), 5 = TMA-staged
+                        tiles, 2 CTAs per SM.  3D: 0 = point tiles, 1 =
+                        streaming, 2-5 = the TMA plane pipeline               */
   int tile_z;        /* 2D streaming kernel: rows per CTA (32, 64 or 128)     */
   int tile_x;        /* 2D streaming kernel: columns walked per CTA (>= 1)    */
-  int tile_y;        /* 3D streaming kernel: y planes marched per CTA (>= 1)  */
+  int tile_y;        /* 3D: y planes marched per CTA (streaming) or taken per
+                        work unit (plane pipeline), >= 1; with the pipeline
+                        the default, 32, lets the library choose              */
   int graph_chunk;   /* time steps per captured CUDA graph (>= 1)             */
-  int use_graph;     /* 0: launch every step directly                         */
+  int use_graph;     /* 0: launch every step directly (never on the chip)     */
 } sw_tuning;
 int sw_ctx_set_tuning(sw_ctx *ctx, const sw_tuning *t);
 int sw_ctx_get_tuning(const sw_ctx *ctx, sw_tuning *t);

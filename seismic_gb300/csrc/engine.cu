@@ -73,11 +73,12 @@ int sw_ctx_reset_stats(sw_ctx *c) {
 }
 int sw_ctx_set_tuning(sw_ctx *c, const sw_tuning *t) {
   if (!c || !t) return SW_BAD_PARAM;
-  if (t->step_kernel < 0 || t->step_kernel > 4 || t->graph_chunk < 1 || t->tile_x < 1 ||
+  if (t->step_kernel < 0 || t->step_kernel > 5 || t->graph_chunk < 1 || t->tile_x < 1 ||
       t->tile_y < 1 ||
       (t->tile_z != 32 && t->tile_z != 64 && t->tile_z != 128))
     return swave::fail(c, SW_BAD_PARAM, "invalid tuning");
-  c->run_opts.tile.stream2d = t->step_kernel;
+  c->run_opts.tile.stream2d = t->step_kernel == 5 ? 2 : t->step_kernel;
+  c->run_opts.onchip = t->step_kernel != 5;
   c->run_opts.tile.stream3d = t->step_kernel == 0 ? 0 : t->step_kernel == 1 ? 1 : 2;
   c->run_opts.tile.ty = t->tile_y;
   c->run_opts.tile.tz = t->tile_z;
@@ -89,7 +90,7 @@ int sw_ctx_set_tuning(sw_ctx *c, const sw_tuning *t) {
 
 int sw_ctx_get_tuning(const sw_ctx *c, sw_tuning *t) {
   if (!c || !t) return SW_BAD_PARAM;
-  t->step_kernel = c->run_opts.tile.stream2d;
+  t->step_kernel = c->run_opts.onchip ? c->run_opts.tile.stream2d : 5;
   t->tile_z = c->run_opts.tile.tz;
   t->tile_x = c->run_opts.tile.tx;
   t->tile_y = c->run_opts.tile.ty;

@@ -216,3 +216,38 @@ def test_profiled_bytes_are_of_the_timed_kernel(fake):
         st = c.stats()
         assert fake.kernels("k_oc_image") and st["step_kernel_timed"] == 2 * g.nt
         assert st["step_bytes"] == steps + saved
+
+
+def test_step_kernel_5_stays_off_the_chip(fake):
+    """step_kernel 5 is the per-step tile kernel in the form that large grids
+    take: a captured graph, receiver samples of 4 steps per launch."""
+    g, vel, sou, rec, w = case2d(nz=60, nx=80, nt=60)
+    with fake.context() as c:
+        assert c.tuning()["step_kernel"] == 2          # the default: on the chip
+        c.modeling(g, vel, sou, w, rec)
+        assert fake.kernels("k_onchip2d") and not fake.kernels("k_bstep2d_t")
+        fake.reset()
+        c.set_tuning(step_kernel=5)
+        assert c.tuning()["step_kernel"] == 5
+        c.modeling(g, vel, sou, w, rec)
+        assert fake.kernels("k_bstep2d_t") and not fake.kernels("k_onchip2d")
+        assert len(fake.kernels("graph")) == 4
+        assert {k[1][1] for k in fake.kernels("k_bextract")} == {4}
+        fake.reset()
+        c.set_tuning(graph_chunk=7)                     # another setting keeps it
+        c.modeling(g, vel, sou, w, rec)
+        assert not fake.kernels("k_onchip2d")
+        assert {k[1][1] for k in fake.kernels("k_bextract")} == {4, 3}
+        fake.reset()
+        c.set_tuning(step_kernel=2)
+        c.modeling(g, vel, sou, w, rec)
+        assert fake.kernels("k_onchip2d")
+        for bad in (-1, 6):
+            with pytest.raises(sw.SwaveError):
+                c.set_tuning(step_kernel=bad)
+        g3, vel3, sou3, rec3, w3 = case3d(nt=4)
+        for k in (2, 5):
+            fake.reset()
+            c.set_tuning(step_kernel=k)
+            c.modeling(g3, vel3, sou3, w3, rec3)
+            assert fake.kernels("k_bstep3d_t")
