@@ -4,7 +4,8 @@ the number of shots per launch.
 Candidates are timed on a truncated copy of the real batch (same windows,
 same number of shots in flight, a few dozen time steps of both the forward
 and the backward phase); the fastest is cached per (device, padded-grid
-bucket, shots per batch) in a JSON file under the user's cache directory.
+bucket, shots per batch, KERNELS) in a JSON file under the user's cache
+directory.
 With `batch="auto"` the shots per launch are chosen first (each candidate
 batch size runs the same sample of shots, in as many launches as it needs,
 with the current launch shape), then the launch shape at that batch size.
@@ -20,6 +21,13 @@ from typing import Callable, Iterable
 
 DEFAULT_CACHE = os.path.join(os.environ.get("XDG_CACHE_HOME", os.path.expanduser("~/.cache")),
                              "seismic_gb300", "tuning.json")
+
+
+# The set of step kernels that entries of the cache chose from; raised with
+# every kernel or rule that changes which choice is the fastest.  Entries of
+# another set are timed again: one from before the on-chip path (set 2) may
+# name a per-step kernel, which keeps shots off the chip.
+KERNELS = 2
 
 
 def candidates(two_d: bool = True) -> list[dict]:
@@ -140,7 +148,8 @@ def tune_batch(ctx, model, vel, wavelet, shots, steps: int = 48,
     widths = [int(np.ptp(np.asarray(s["rec"])[:, 1]) / g.dx) + 1 for s in sample]
     n2p = max(widths) + 2 * g.ntaper + 8
     n3p = 1 if g.twoD else g.ny + 2 * g.ntaper + 8
-    key = cache_key(_device_name(ctx, device_name), n1p, n2p, n3p, len(shots)) + "|batch"
+    key = (cache_key(_device_name(ctx, device_name), n1p, n2p, n3p, len(shots)) +
+           f"|k{KERNELS}|batch")
     cache = load_cache(cache_path) if cache_path else {}
     if key in cache and not force:
         return cache[key]
@@ -188,7 +197,7 @@ def tune_rtm(ctx, model, vel, wavelet, shots, steps: int = 48, batch: int | str 
     widths = [int(np.ptp(np.asarray(s["rec"])[:, 1]) / g.dx) + 1 for s in sample]
     n2p = max(widths) + 2 * g.ntaper + 8
     n3p = 1 if g.twoD else g.ny + 2 * g.ntaper + 8
-    key = cache_key(_device_name(ctx, device_name), n1p, n2p, n3p, batch)
+    key = cache_key(_device_name(ctx, device_name), n1p, n2p, n3p, batch) + f"|k{KERNELS}"
     cache = load_cache(cache_path) if cache_path else {}
     if key in cache and not force:
         ctx.set_tuning(**cache[key]["tuning"])

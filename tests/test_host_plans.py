@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 import seismic_gb300 as sw
+from seismic_gb300 import autotune
 from tests.cases import case2d, case3d
 from tests.fakecuda import Fake
 
@@ -251,3 +252,23 @@ def test_step_kernel_5_stays_off_the_chip(fake):
             c.set_tuning(step_kernel=k)
             c.modeling(g3, vel3, sou3, w3, rec3)
             assert fake.kernels("k_bstep3d_t")
+
+
+def test_tuning_cached_for_other_kernels_is_not_taken(fake, tmp_path):
+    """A cache written before the present set of step kernels (its keys name no
+    set) neither keeps shots off the chip nor fixes the shots per launch."""
+    g, vel, sou, rec, w = case2d(nz=60, nx=80, nt=40)
+    shots = [{"sou": sou, "rec": rec, "data": np.zeros((len(rec), g.nt), np.float32)}] * 2
+    path = str(tmp_path / "tuning.json")
+    n1p, n2p = g.nz + 2 * g.ntaper + 8, g.nx + 2 * g.ntaper + 8
+    key = autotune.cache_key("dev", n1p, n2p, 1, 2)
+    old = {"step_kernel": 3, "tile_z": 64, "tile_x": 64, "tile_y": 32, "graph_chunk": 16,
+           "use_graph": 1}
+    autotune.save_cache({key: {"tuning": old}, key + "|batch": {"batch": 77}}, path)
+    with fake.context() as c:
+        got = autotune.tune_rtm(c, g, vel, w, shots, steps=20, batch="auto", cache_path=path,
+                                device_name="dev")
+        assert got["batch"] in (1, 2) and got["tried"] == len(autotune.candidates(True))
+        again = autotune.tune_rtm(c, g, vel, w, shots, steps=20, batch="auto", cache_path=path,
+                                  device_name="dev")
+        assert again == got                             # its own entries are
