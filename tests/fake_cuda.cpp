@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <cuda.h>
 
+#include <unistd.h>
+
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
@@ -216,6 +218,7 @@ cudaError_t cudaGetSymbolAddress(void **p, const void *s) {
 }
 cudaError_t cudaGetDriverEntryPointByVersion(const char *, void **p, unsigned, unsigned long long,
                                              cudaDriverEntryPointQueryResult *r) {
+  usleep(200000);   // a slow lookup: a second thread asks meanwhile
   *p = (void *)encode;
   if (r) *r = cudaDriverEntryPointSuccess;
   return cudaSuccess;
