@@ -97,7 +97,8 @@ typedef enum sw_imaging {
   SW_IMG_BORN = 4,   /* Injection_Born                           (Imaging.f90:747) */
   SW_IMG_AFWI_RHO = 5 /* Imaging_condition_AFWI_RHOVP_from_memory (Imaging.f90:424):
                          the velocity gradient into image, the density
-                         gradient into image2; needs rho (withRho)    */
+                         gradient into image2; needs rho (withRho) and
+                         nz, nx >= 2                                  */
 } sw_imaging;
 
 /* One propagation = one call of propagator_acoustic. */

@@ -500,6 +500,9 @@ int run_phases(sw_ctx *c, std::vector<PhaseShot> &shots, const RunOpts &opt) {
       return fail(c, SW_BAD_PARAM, "image buffers missing");
     if (S.imaging == SW_IMG_AFWI_RHO && (!S.image2 || !S.rho_on))
       return fail(c, SW_BAD_PARAM, "SW_IMG_AFWI_RHO needs rho and image2");
+    // Its differences along z and x take two points of the snapshot.
+    if (S.imaging == SW_IMG_AFWI_RHO && (g.nz < 2 || g.nx < 2))
+      return fail(c, SW_BAD_PARAM, "SW_IMG_AFWI_RHO needs nz and nx of at least 2");
     if (S.imaging == SW_IMG_BORN && !S.ref) return fail(c, SW_BAD_PARAM, "reflectivity missing");
     max_steps = std::max(max_steps, S.nsteps);
     step_tiles[b + 1] = step_tiles[b] + step_ctas(G[b], tile);

@@ -272,3 +272,26 @@ def test_tuning_cached_for_other_kernels_is_not_taken(fake, tmp_path):
         again = autotune.tune_rtm(c, g, vel, w, shots, steps=20, batch="auto", cache_path=path,
                                   device_name="dev")
         assert again == got                             # its own entries are
+
+
+@pytest.mark.parametrize("nz,nx,ny,ok", [(1, 20, 1, False), (20, 1, 1, False), (2, 2, 1, True),
+                                         (9, 1, 8, False), (1, 9, 8, False), (9, 9, 1, True)])
+def test_density_imaging_of_a_single_row_or_column_is_refused(fake, nz, nx, ny, ok):
+    """The differences of SW_IMG_AFWI_RHO on one row or column would start
+    before the snapshots' memory."""
+    g = sw.make_genpar(nz, nx, ny, dz=10.0, dx=10.0, dy=10.0, dt=1e-3, nt=12, ntaper=10,
+                       twoD=ny == 1)
+    vel = np.full((ny, nx, nz), 2000.0, np.float32)
+    z = lambda: np.zeros(vel.size, np.float32)
+    d = sw.SwPropDesc()
+    d.g, d.tmin, d.tmax, d.tstep, d.imaging = g, g.nt, 1, -1, sw.IMG_AFWI_RHO
+    with fake.context() as c:
+        call = lambda: c.propagate(d, vel, wave=np.zeros(3 * vel.size, np.float32), image=z(),
+                                   illum=z(), image2=z(), rho=vel)
+        if ok:
+            call()
+        else:
+            with pytest.raises(sw.SwaveError) as e:
+                call()
+            assert e.value.code == sw.SW_BAD_PARAM
+            assert not fake.kernels("k_brho") and not fake.kernels("k_bstep")
