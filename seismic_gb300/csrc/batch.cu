@@ -468,7 +468,8 @@ __global__ void k_brho_grad(BatchTables t, int s_off) {
 // wave: 64 x 32 tiles with everything staged, two blocks per SM: 24.7 us per
 // step (and 8.2 for the edges); three blocks, the update's inputs from
 // registers: 22.0, the SMs busy for 69 % of it (2.1 waves); 32 x 32 tiles,
-// four blocks: 21 with the edges.
+// four blocks: 21 with the edges (64 registers, at which it spills 20 bytes
+// and loads 52).
 // sz and sx never go through HBM: 32 bytes per point (u2, delp, v, rho, u1,
 // u0, u_1 read, u3 written) instead of the two passes' 52.
 // ---------------------------------------------------------------------------
@@ -1292,7 +1293,8 @@ __global__ void k_bterms(BatchTables t, int s_off, int sub) {
 // first n_term blocks form the injection terms of step s + 1, the next
 // n_edge blocks the absorbing edges of step s (edges3d), the rest its
 // snapshot saves and imaging.  The parts touch nothing in common: the edges
-// write u3 and read u2 and u1, the snapshots read u2.  Each is bound by
+// write u3 and read u2 and u1, the snapshots read u2.  The lines take 128
+// registers, so all parts run at 16 warps per SM.  Each is bound by
 // memory latency when it runs alone (240 x 440 x 440: z, x and y lines 33,
 // 15 and 12 us one after the other; 140 x 240 x 240: terms 7, snapshots 7 to
 // 27, lines 14, 10 and 8 us).

@@ -217,7 +217,8 @@ __device__ __noinline__ float higdon_corner(const ShotDev &S, int i, int j, int 
 // and starts from two cells that an earlier one may have written.  So here a
 // z line of the outer 4 columns or planes, and an x line of the outer
 // planes, is left out (no later step reads the padding cells which only they
-// wrote), and a line that starts in a corner forms those two cells itself
+// wrote, and calls whose receivers or outputs do take the lines in order), and
+// a line that starts in a corner forms those two cells itself
 // (higdon_corner): the lines are independent.
 __device__ __forceinline__ void edges3d(const ShotDev &S, int s, int q) {
   const Geom &g = S.g;
